@@ -7,6 +7,7 @@
   run(state)       one pass; returns the path's outputs
   work(case)       bytes and operations one pass cannot do without
   tolerance(case)  how far another correct implementation of the same precision may be off
+  exact(case, s)   what run() returns for the inputs of seed s, in plain torch and 64 bits
 
 The model is the framework's own benchmark model, Llama-2-7B's architecture with int4 linears (group 128), random
 weights: zero-mean nibbles and scales that keep activations in range, as a trained checkpoint has them.
@@ -302,3 +303,82 @@ def tolerance(case):
     if kind == "custom_ir":
         return {"rel": 2e-6, "max": 2e-5} if f32 else {"rel": 8e-4, "max": 3e-3}
     return {"rel": 0.03, "max": 0.2}
+
+
+# ---- the same results in 64 bits ---------------------------------------------------------------------------
+
+def _dequant(q, s):
+    """Weights [K, N] in 64 bits from packed nibbles [K/8, N] and group scales [K/128, N], nothing rounded on the way."""
+    w = torch.stack([((q >> (4 * j)) & 15) - 8 for j in range(8)], dim=1).view(-1, q.shape[1]).double()
+    return w.view(s.shape[0], GROUP, -1).mul_(s.double()[:, None]).view(w.shape)
+
+
+def _rms64(x, w):
+    return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + 1e-6) * w.double()
+
+
+def _rope64(x, pos, inv_freq):
+    """x [T, H, D] rotated by halves at the positions pos [T]; angles as float32 products, which is what defines them."""
+    ang = (pos.float()[:, None] * inv_freq[None]).double()[:, None]
+    half = x.shape[-1] // 2
+    return x * ang.cos() + torch.cat([-x[..., half:], x[..., :half]], -1) * ang.sin()
+
+
+def _attend64(q, k, v, first):
+    """Rows of q [T, H, D] at positions first, first + 1, ... over the cache rows k, v [S, H, D] up to their own."""
+    later = torch.arange(k.shape[0], device="cuda")[None] > torch.arange(first, first + q.shape[0], device="cuda")[:, None]
+    heads = []
+    for h in range(q.shape[1]):
+        heads.append(torch.softmax((q[:, h] @ k[:, h].T / math.sqrt(q.shape[2])).masked_fill_(later, -math.inf), -1) @ v[:, h])
+    return torch.stack(heads, 1)
+
+
+def _model64(case, seed):
+    cfg = LlamaConfig(n_layers=case["layers"], max_seq=MAX_SEQ)
+    ckpt, n = _Checkpoint(cfg), case["prompt"]
+    toks = torch.from_numpy(synth_prompt(cfg, n + case.get("steps", 0), int(seed))).cuda().long()
+    inv_freq, pos = torch.from_numpy(make_inv_freq(HEAD, 10000.0)).cuda(), torch.arange(len(toks), device="cuda")
+    on = lambda w, *keys: [torch.from_numpy(w[k]).cuda() for k in keys]  # noqa: E731
+    embed, head, final = on(ckpt.globals(), "embed", "lm_head", "final_norm")
+    x, ks, vs = embed[toks].double(), [], []
+    for l in range(case["layers"]):
+        w = ckpt.layer(l)
+        mm = lambda a, key: a @ _dequant(*on(w, key + "_q", key + "_s"))  # noqa: E731
+        v, q, k = mm(_rms64(x, *on(w, "att_norm")), "vqk").view(-1, 3, HEADS, HEAD).unbind(1)
+        q, k = _rope64(q, pos, inv_freq), _rope64(k, pos, inv_freq)
+        x = x + mm(_attend64(q, k, v, 0).reshape(-1, DIM), "o")
+        ks.append(k.reshape(-1, DIM))
+        vs.append(v.reshape(-1, DIM))
+        h = _rms64(x, *on(w, "ffn_norm"))
+        x = x + mm(torch.nn.functional.silu(mm(h, "gate")) * mm(h, "up"), "down")
+    logits = lambda row: _rms64(row, final) @ head.double().T  # noqa: E731
+    out = {"k_cache": torch.stack(ks), "v_cache": torch.stack(vs)}
+    if case["kind"] == "chat":
+        out["first_logits"] = logits(x[n - 1])
+    out["logits"] = logits(x[-1])
+    return out
+
+
+def exact(case, seed):
+    kind = case["kind"]
+    if kind in ("chat", "prefill"):
+        return _model64(case, seed)
+    st = prepare(case, seed)
+    if kind == "export":
+        return st["x"].double() @ _dequant(st["q"], st["s"])
+    if kind in ("projections", "gemm"):
+        return [x.double() @ _dequant(q, s) for x, q, s in st["calls"]]
+    if kind == "sample_layer":
+        at, x, pos = torch.tensor([st["pos"]], device="cuda"), st["x"].double(), st["pos"]
+        v, q, k = (_rms64(x, st["att_norm"]) @ _dequant(*st["vqk"])).view(3, 1, HEADS, HEAD)
+        kc, vc = st["kc"].double(), st["vc"].double()
+        q, kc[pos], vc[pos] = _rope64(q, at, st["inv_freq"]), _rope64(k, at, st["inv_freq"]).view(DIM), v.view(DIM)
+        cache = [c[:pos + 1].view(-1, HEADS, HEAD) for c in (kc, vc)]
+        x = x + _attend64(q, *cache, pos).view(DIM) @ _dequant(*st["o"])
+        h = _rms64(x, st["ffn_norm"])
+        return [x + (torch.nn.functional.silu(h @ _dequant(*st["gate"])) * (h @ _dequant(*st["up"]))) @ _dequant(*st["down"]), kc, vc]
+    if kind == "elementwise":
+        return [torch.sigmoid(st["data"].double()), _rms64(st["hidden"].double(), st["weight"]),
+                _rope64(st["heads"].double(), st["pos"], st["inv_freq"]), torch.softmax(st["scores"].double(), -1)]
+    y = torch.nn.functional.layer_norm(st["x"].double(), (case["cols"],), st["g"].double(), st["b"].double(), 1e-5)
+    return [y, torch.nn.functional.gelu(y.view(-1), approximate="tanh")]
