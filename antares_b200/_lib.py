@@ -58,8 +58,10 @@ SIGNATURES = {
     "ab200_rmsnorm_vsum": [_vp, _vp, _vp, _vp, _sz, _f, _f, _i, _vp],
     "ab200_rmsnorm": [_vp, _i, _vp, _vp, _i, _i, _f, _vp],
     "ab200_rope": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
+    "ab200_rope_at": [_vp, _vp, _i, _vp, _i, _i, _i, _vp],
     "ab200_softmax": [_vp, _vp, _i, _i, _i, _vp],
     "ab200_attention_decode": [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _l, _f, _i, _vp],
+    "ab200_attention_decode_at": [_vp, _vp, _vp, _vp, _i, _i, _i, _l, _vp, _i, _vp],
     "ab200_embed_lookup": [_vp, _vp, _vp, _i, _i, _vp],
     "ab200_rope_kv_store": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _l, _i, _vp],
     "ab200_attention_fused": [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _l, _i, _f, _vp],
@@ -113,6 +115,23 @@ def load():
         L.ab200_w4a16_gemv_emulation_scratch_bytes.argtypes = []
         _lib = L
     return _lib
+
+
+_fast = None
+
+
+def fast():
+    """The native front end (csrc/fastcall.cpp), its entry points bound.  Raises ImportError if it has not been built."""
+    global _fast
+    if _fast is None:
+        L = load()
+        try:
+            from . import _fastcall
+        except ImportError as e:
+            raise ImportError("antares_b200/_fastcall.so: %s; run `python -m antares_b200.build`" % e)
+        _fastcall.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in SIGNATURES})
+        _fast = _fastcall
+    return _fast
 
 
 def call(name, *args):

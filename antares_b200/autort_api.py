@@ -22,6 +22,7 @@ import torch
 
 from . import ir as _ir
 from . import ops as _ops
+from ._lib import fast
 
 RMS_EPS = 1e-6  # epsilon of the built-in rmsnorm ops (the reference's value is inside its closed wheel)
 
@@ -111,6 +112,19 @@ class NativeModules:
 
 
 _DT_NAME = {torch.float16: "float16", torch.float32: "float32"}
+_DT_CODE = {"float16": 0, "float32": 1, "int32": 2}
+
+
+def _program(match, kind, order=(), x=0, q=0, stages=(), consts=(), mats=(), cols=()):
+    """The exported op as the native front end runs it (csrc/fastcall.cpp), or None where it does not; stages:
+    [(kind, postfix program)]; mats / cols: names of the operands in the program's order."""
+    index = {s.name: i for i, s in enumerate(match.inputs)}
+    if len(match.inputs) > 8 or any(s.dtype not in _DT_CODE for s in match.inputs):
+        return None
+    flat = [oa for _, prog in stages for oa in prog]
+    return fast().program(kind, [(_DT_CODE[s.dtype], list(s.dims), [0 if d is None else 1 for d in s.dyn]) for s in match.inputs], list(order), x, q,
+                          [int(o) for o, _ in flat], [int(a) for _, a in flat], [len(prog) for _, prog in stages], [int(k) for k, _ in stages],
+                          [float(c) for c in consts], [index[n] for n in mats], [index[n] for n in cols])
 
 
 def export(ir, inputs, config=None, name=None):
@@ -119,8 +133,15 @@ def export(ir, inputs, config=None, name=None):
     if match.kind in ("w4a16", "sigmoid", "softmax"):
         pr = match.params
         native = NativeModules(ir, match.inputs, match.output)
+        names = [s.name for s in match.inputs]
+        state = []  # the native front end's program, made by the first call
 
         def fn(*tensors, out=None, extra=None):
+            plain = out is None and len(tensors) == len(names)
+            if plain and state:
+                y = state[0] and fast().run(state[0], *tensors)
+                if y is not None:
+                    return y
             t, out = _split_call(match, tensors, out)
             ordered = [t[s.name] for s in match.inputs]
             for a in ordered:
@@ -137,12 +158,23 @@ def export(ir, inputs, config=None, name=None):
             elif out.numel() != int(torch.Size(shape).numel()) or out.dtype != x.dtype or not out.is_contiguous():
                 raise ValueError("%s: out must be a contiguous %s tensor of %d elements" % (match.name, x.dtype, torch.Size(shape).numel()))
             native.forward(ordered, out.view(shape) if out.shape != shape else out, _DT_NAME[x.dtype])
+            if not state:
+                state.append(_program(match, 0 if match.kind == "w4a16" else 1, native.order, names.index(pr["x"]), names.index(pr["qweight"]) if match.kind == "w4a16" else 0))
+            if plain and state[0]:
+                fast().known(state[0], native.keys[(tuple(tuple(a.shape) for a in ordered), tuple(shape))], *ordered)
             return out
         fn.native = native
     elif match.kind == "eltwise":
         pr = match.params
+        state = []
 
         def fn(*tensors, out=None, extra=None):
+            if out is None and len(tensors) == len(match.inputs):
+                if not state:
+                    state.append(_program(match, 2, stages=[(0, pr["program"])], consts=pr["consts"], mats=pr["inputs"]))
+                y = state[0] and fast().run(state[0], *tensors)
+                if y is not None:
+                    return y
             t, out = _split_call(match, tensors, out)
             ins = [t[n] for n in pr["inputs"]]
             shape = ins[0].shape
@@ -156,8 +188,15 @@ def export(ir, inputs, config=None, name=None):
             return _ops.eltwise_program(pr["program"], pr["consts"], ins, out=out)
     elif match.kind == "rowprog":
         rp = match.params
+        state = []
 
         def fn(*tensors, out=None, extra=None):
+            if out is None and len(tensors) == len(match.inputs):
+                if not state:
+                    state.append(_program(match, 3, stages=rp["stages"], consts=rp["consts"], mats=rp["mats"], cols=rp["cols"]))
+                y = state[0] and fast().run(state[0], *tensors)
+                if y is not None:
+                    return y
             t, out = _split_call(match, tensors, out)
             return _ops.row_program(rp, [t[n] for n in rp["mats"]], [t[n] for n in rp["cols"]], out=out)
     else:  # pragma: no cover - recognise() raises first
@@ -174,6 +213,10 @@ def _rmsnorm(dtype):
     def fn(x, vsum, weight, out=None, extra=None):
         if not extra:
             raise TypeError("rmsnorm needs extra=[1/N]")
+        if out is None and x.dtype == dtype:
+            y = fast().rmsnorm_vsum(x, vsum, weight, extra[0], RMS_EPS)
+            if y is not None:
+                return y
         if x.dtype != dtype or weight.dtype != dtype:
             raise TypeError("rmsnorm_%s: x and weight must be %s" % ("f32" if dtype == torch.float32 else "f16", dtype))
         return _ops.rmsnorm_vsum(x.contiguous(), vsum.reshape(1).float(), weight.contiguous(), float(extra[0]), RMS_EPS, out=out)
@@ -181,9 +224,14 @@ def _rmsnorm(dtype):
 
 
 def _rotary(dtype):
+    code = 0 if dtype == torch.float16 else 1
+
     def fn(x, inv_freq, out=None, extra=None):
         if not extra:
             raise TypeError("rotary needs extra=[pos]")
+        y = fast().rope_at(code, x, inv_freq, out, int(extra[0]))  # the position is a host value: no copy to the device
+        if y is not None:
+            return y
         if x.dtype != dtype:
             raise TypeError("rotary: x must be %s" % dtype)
         H = x.shape[0]
@@ -196,7 +244,13 @@ def _rotary(dtype):
 
 
 def _attention(dtype):
+    code = 0 if dtype == torch.float16 else 1
+
     def fn(q, k, v, att_f, out=None, extra=None):
+        if out is None:
+            y = fast().attend_at(code, q, k, v, att_f)  # att_f is read on the device: no synchronisation
+            if y is not None:
+                return y
         if q.dtype != dtype:
             raise TypeError("attention: q must be %s" % dtype)
         H, D = q.shape

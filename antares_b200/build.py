@@ -1,4 +1,5 @@
-"""Builds antares_b200/libantares_b200.so from csrc/*.cu with nvcc for sm_100a (in-tree, no JIT cache).
+"""Builds antares_b200/libantares_b200.so from csrc/*.cu with nvcc for sm_100a, and antares_b200/_fastcall.so, the
+Python front end's native part, from csrc/fastcall.cpp with g++ (both in-tree, no JIT cache).
 
   python -m antares_b200.build [--force] [--verbose]
 """
@@ -10,6 +11,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libantares_b200.so")
+FAST_SRC, FAST = os.path.join(CSRC, "fastcall.cpp"), os.path.join(HERE, "_fastcall.so")
 
 NVCC_FLAGS = ["-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
               "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
@@ -34,7 +36,23 @@ def up_to_date():
     return all(os.path.getmtime(d) <= t for d in deps)
 
 
+def build_fastcall(force=False):
+    if not force and os.path.exists(FAST) and os.path.getmtime(FAST_SRC) <= os.path.getmtime(FAST):
+        return FAST
+    import sysconfig
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
+    subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+                           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-I" + sysconfig.get_paths()["include"],
+                           "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                           "-I" + os.path.join(cuda, "include"), FAST_SRC, "-o", FAST, "-L" + os.path.join(root, "lib"),
+                           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    return FAST
+
+
 def build(force=False, verbose=False):
+    build_fastcall(force)
     if not force and up_to_date():
         return LIB
     objs = []

@@ -41,14 +41,16 @@ template <typename T>
 __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(const T *__restrict__ q, const T *__restrict__ kc,
                                                                       const T *__restrict__ vc, T *__restrict__ out,
                                                                       const int32_t *__restrict__ seq_len_dev, int seq_len_add,
-                                                                      int max_seq, long kv_stride, float scale, KvPages pages) {
+                                                                      int max_seq, long kv_stride, float scale, const float *__restrict__ scale_dev,
+                                                                      KvPages pages) {
   extern __shared__ __align__(16) float att_smem[];
   float *p = att_smem;                // [max_seq]
   float *red = att_smem + max_seq;    // [16][128]
   __shared__ float sh[32];
   const int h = blockIdx.x;
   // blockIdx.y = query row of a causal prefill: row r sees r more cache rows than row 0
-  int S = *seq_len_dev + seq_len_add + (int)blockIdx.y;
+  int S = (seq_len_dev ? *seq_len_dev : 0) + seq_len_add + (int)blockIdx.y;
+  if (scale_dev) scale = *scale_dev;
   S = S < 0 ? 0 : (S > max_seq ? max_seq : S);
   q += (size_t)blockIdx.y * gridDim.x * ATT_D;
   out += (size_t)blockIdx.y * gridDim.x * ATT_D;
@@ -343,11 +345,9 @@ __global__ void __launch_bounds__(DG_THREADS) dense_gemv_kernel(const __half *__
 
 using namespace ab200;
 
-extern "C" int ab200_attention_decode(const void *q_f16, const void *k_cache_f16, const void *v_cache_f16, void *out_f16,
-                                      const int32_t *seq_len_dev, int seq_len_add, int max_seq, int H, int D, long kv_stride,
-                                      float scale, int dtype, void *stream) {
-  clear_error();
-  AB200_REQUIRE(q_f16 && k_cache_f16 && v_cache_f16 && out_f16 && seq_len_dev, "attention_decode: null pointer");
+static int attention_decode_impl(const void *q_f16, const void *k_cache_f16, const void *v_cache_f16, void *out_f16,
+                                 const int32_t *seq_len_dev, int seq_len_add, int max_seq, int H, int D, long kv_stride,
+                                 float scale, const float *scale_dev, int dtype, void *stream) {
   AB200_REQUIRE(D == ATT_D, "attention_decode: head size %d is not the built size %d", D, ATT_D);
   AB200_REQUIRE(H > 0 && max_seq > 0 && kv_stride >= (long)H * D && kv_stride % 8 == 0, "attention_decode: bad shape H=%d max_seq=%d kv_stride=%ld", H, max_seq, kv_stride);
   AB200_REQUIRE(aligned16(q_f16) && aligned16(k_cache_f16) && aligned16(v_cache_f16) && aligned16(out_f16),
@@ -359,18 +359,33 @@ extern "C" int ab200_attention_decode(const void *q_f16, const void *k_cache_f16
       AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attention_decode_kernel<__half><<<H, ATT_THREADS, smem, (cudaStream_t)stream>>>((const __half *)q_f16, (const __half *)k_cache_f16,
                                                                                    (const __half *)v_cache_f16, (__half *)out_f16, seq_len_dev,
-                                                                                   seq_len_add, max_seq, kv_stride, scale, KvPages{nullptr, 0});
+                                                                                   seq_len_add, max_seq, kv_stride, scale, scale_dev, KvPages{nullptr, 0});
   } else if (dtype == AB200_F32) {
     if (smem > 48 * 1024)
       AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     attention_decode_kernel<float><<<H, ATT_THREADS, smem, (cudaStream_t)stream>>>((const float *)q_f16, (const float *)k_cache_f16,
                                                                                   (const float *)v_cache_f16, (float *)out_f16, seq_len_dev,
-                                                                                  seq_len_add, max_seq, kv_stride, scale, KvPages{nullptr, 0});
+                                                                                  seq_len_add, max_seq, kv_stride, scale, scale_dev, KvPages{nullptr, 0});
   } else {
     return fail(AB200_EINVAL, "attention_decode: unknown dtype %d", dtype);
   }
   AB200_CHECK_LAUNCH("attention_decode");
   return AB200_OK;
+}
+
+extern "C" int ab200_attention_decode(const void *q_f16, const void *k_cache_f16, const void *v_cache_f16, void *out_f16,
+                                      const int32_t *seq_len_dev, int seq_len_add, int max_seq, int H, int D, long kv_stride,
+                                      float scale, int dtype, void *stream) {
+  clear_error();
+  AB200_REQUIRE(q_f16 && k_cache_f16 && v_cache_f16 && out_f16 && seq_len_dev, "attention_decode: null pointer");
+  return attention_decode_impl(q_f16, k_cache_f16, v_cache_f16, out_f16, seq_len_dev, seq_len_add, max_seq, H, D, kv_stride, scale, nullptr, dtype, stream);
+}
+
+extern "C" int ab200_attention_decode_at(const void *q, const void *k_cache, const void *v_cache, void *out, int seq_len, int H, int D, long kv_stride,
+                                         const float *scale_dev, int dtype, void *stream) {
+  clear_error();
+  AB200_REQUIRE(q && k_cache && v_cache && out && scale_dev, "attention_decode_at: null pointer");
+  return attention_decode_impl(q, k_cache, v_cache, out, nullptr, seq_len, seq_len, H, D, kv_stride, 0.f, scale_dev, dtype, stream);
 }
 
 extern "C" int ab200_dense_gemv(const void *x_f16, const void *w_f16, float *logits_f32, int K, int N, void *stream) {
@@ -454,7 +469,7 @@ static int attention_prefill_impl(const void *q_f16, const void *k_cache_f16, co
   if (smem > 200 * 1024) return fail(AB200_EUNSUPPORTED, "attention_prefill: max_seq=%d exceeds the shared-memory score buffer", max_seq);
   if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   attention_decode_kernel<__half><<<dim3(H, rows), ATT_THREADS, smem, (cudaStream_t)stream>>>(
-      (const __half *)q_f16, (const __half *)k_cache_f16, (const __half *)v_cache_f16, (__half *)out_f16, pos0_dev, 1, max_seq, kv_stride, scale,
+      (const __half *)q_f16, (const __half *)k_cache_f16, (const __half *)v_cache_f16, (__half *)out_f16, pos0_dev, 1, max_seq, kv_stride, scale, nullptr,
       KvPages{page_table, page_table ? page_shift_of(page_rows) : 0});
   AB200_CHECK_LAUNCH("attention_prefill");
   return AB200_OK;

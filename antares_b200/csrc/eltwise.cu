@@ -159,7 +159,7 @@ __global__ void rmsnorm_vsum_kernel(const T *__restrict__ x, const float *__rest
 // and walks the heads with a stride of the CTA.
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS) rope_kernel(const T *__restrict__ x, const float *__restrict__ inv_freq,
-                                                          const int32_t *__restrict__ pos, T *__restrict__ out,
+                                                          const int32_t *__restrict__ pos, int pos_host, T *__restrict__ out,
                                                           int H, int D) {
   __shared__ float sh_c[ROW_THREADS * 8], sh_s[ROW_THREADS * 8];  // D / 2 <= 8 * ROW_THREADS (the host checks D / 16 <= ROW_THREADS)
   const size_t row = blockIdx.x;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(ROW_THREADS) rope_kernel(const T *__restrict__
   }
   for (int j = threadIdx.x; j < half; j += ROW_THREADS) {
     float sv, cv;
-    sincosf((float)pos[row] * inv_freq[j], &sv, &cv);
+    sincosf((float)(pos ? pos[row] : pos_host) * inv_freq[j], &sv, &cv);
     sh_s[j] = sv;
     sh_c[j] = cv;
   }
@@ -454,18 +454,28 @@ extern "C" int ab200_rmsnorm(const void *x, int x_dtype, const void *weight_f16,
   return AB200_OK;
 }
 
+static int rope_launch(const void *x, const float *inv_freq, const int32_t *pos, int pos_host, void *out, int rows, int H, int D, int dtype, void *stream) {
+  AB200_REQUIRE(D > 0 && D % 16 == 0 && D / 16 <= ROW_THREADS && H > 0 && rows >= 0, "rope: D=%d must be a multiple of 16 (at most %d), H=%d positive", D, ROW_THREADS * 16, H);
+  AB200_REQUIRE(aligned16(x) && aligned16(out), "rope: pointers must be 16-byte aligned");
+  if (rows == 0) return AB200_OK;
+  if (dtype == AB200_F16) rope_kernel<__half><<<rows, ROW_THREADS, 0, (cudaStream_t)stream>>>((const __half *)x, inv_freq, pos, pos_host, (__half *)out, H, D);
+  else if (dtype == AB200_F32) rope_kernel<float><<<rows, ROW_THREADS, 0, (cudaStream_t)stream>>>((const float *)x, inv_freq, pos, pos_host, (float *)out, H, D);
+  else return fail(AB200_EINVAL, "rope: unknown dtype %d", dtype);
+  AB200_CHECK_LAUNCH("rope");
+  return AB200_OK;
+}
+
 extern "C" int ab200_rope(const void *x_f16, const float *inv_freq, const int32_t *pos, void *out_f16, int rows, int H,
                           int D, int dtype, void *stream) {
   clear_error();
   AB200_REQUIRE(x_f16 && inv_freq && pos && out_f16, "rope: null pointer");
-  AB200_REQUIRE(D > 0 && D % 16 == 0 && D / 16 <= ROW_THREADS && H > 0 && rows >= 0, "rope: D=%d must be a multiple of 16 (at most %d), H=%d positive", D, ROW_THREADS * 16, H);
-  AB200_REQUIRE(aligned16(x_f16) && aligned16(out_f16), "rope: pointers must be 16-byte aligned");
-  if (rows == 0) return AB200_OK;
-  if (dtype == AB200_F16) rope_kernel<__half><<<rows, ROW_THREADS, 0, (cudaStream_t)stream>>>((const __half *)x_f16, inv_freq, pos, (__half *)out_f16, H, D);
-  else if (dtype == AB200_F32) rope_kernel<float><<<rows, ROW_THREADS, 0, (cudaStream_t)stream>>>((const float *)x_f16, inv_freq, pos, (float *)out_f16, H, D);
-  else return fail(AB200_EINVAL, "rope: unknown dtype %d", dtype);
-  AB200_CHECK_LAUNCH("rope");
-  return AB200_OK;
+  return rope_launch(x_f16, inv_freq, pos, 0, out_f16, rows, H, D, dtype, stream);
+}
+
+extern "C" int ab200_rope_at(const void *x, const float *inv_freq, int pos, void *out, int H, int D, int dtype, void *stream) {
+  clear_error();
+  AB200_REQUIRE(x && inv_freq && out, "rope_at: null pointer");
+  return rope_launch(x, inv_freq, nullptr, pos, out, 1, H, D, dtype, stream);
 }
 
 extern "C" int ab200_softmax(const void *x, void *out, int rows, int cols, int dtype, void *stream) {

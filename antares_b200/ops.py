@@ -5,7 +5,7 @@ Nothing here computes on the CPU: a CPU tensor is an error, not a fallback.
 import torch
 
 from . import _lib
-from ._lib import F16, F32, call
+from ._lib import F16, F32, call, fast
 
 _DT = {torch.float16: F16, torch.float32: F32}
 
@@ -78,6 +78,10 @@ def _gemm_shapes(x, qweight, scales, group):
 
 def w4a16_gemv(x, qweight, scales, out=None, group=None):
     """out[..., N] = x[..., K] . dequant(qweight, scales); M = x.numel()/K <= 16."""
+    if out is None and group is None:
+        y = fast().w4a16(1, x, qweight, scales)
+        if y is not None:
+            return y
     M, K, N, group = _gemm_shapes(x, qweight, scales, group)
     if out is None:
         out = torch.empty(tuple(x.shape[:-1]) + (N,), dtype=x.dtype, device=x.device)
@@ -99,7 +103,11 @@ def w4a16_gemv_residual(x, qweight, scales, resid, group=None):
 
 
 def w4a16_gemm(x, qweight, scales, out=None, group=None):
-    """Prefill contraction on tensor cores; x [M, K] with M a multiple of 128."""
+    """Prefill contraction on tensor cores."""
+    if out is None and group is None:
+        y = fast().w4a16(2, x, qweight, scales)
+        if y is not None:
+            return y
     Kp, N = qweight.shape
     K = Kp * 8
     M = x.numel() // K
@@ -115,6 +123,10 @@ def w4a16_gemm(x, qweight, scales, out=None, group=None):
 def w4a16_matmul(x, qweight, scales, out=None, group=None):
     """The exported op of samples/05_llama2_7b_int4.py:135-144 for any batch: decode kernel up to
     16 rows, tensor-core kernel above."""
+    if out is None and group is None:
+        y = fast().w4a16(0, x, qweight, scales)
+        if y is not None:
+            return y
     M = x.numel() // (qweight.shape[0] * 8)
     if M <= 16:
         return w4a16_gemv(x, qweight, scales, out, group)
@@ -123,6 +135,9 @@ def w4a16_matmul(x, qweight, scales, out=None, group=None):
 
 def sigmoid(x, out=None):
     if out is None:
+        y = fast().sigmoid(x)
+        if y is not None:
+            return y
         out = torch.empty_like(x)
     call("ab200_sigmoid", _chk(x, "x"), _chk(out, "out", x.dtype), x.numel(), _code(x.dtype), _stream())
     return out
@@ -137,6 +152,10 @@ def rmsnorm_vsum(x, vsum, weight, inv_n, eps=1e-6, out=None):
 
 
 def rmsnorm(x, weight, eps=1e-6, out=None):
+    if out is None:
+        y = fast().rmsnorm(x, weight, eps)
+        if y is not None:
+            return y
     cols = x.shape[-1]
     rows = x.numel() // cols
     if out is None:
@@ -147,6 +166,10 @@ def rmsnorm(x, weight, eps=1e-6, out=None):
 
 
 def rope(x, pos, inv_freq, out=None):
+    if out is None:
+        y = fast().rope(x, pos, inv_freq)
+        if y is not None:
+            return y
     rows, H, D = x.shape
     if out is None:
         out = torch.empty_like(x)
@@ -156,6 +179,10 @@ def rope(x, pos, inv_freq, out=None):
 
 
 def softmax(x, out=None):
+    if out is None:
+        y = fast().softmax(x)
+        if y is not None:
+            return y
     cols = x.shape[-1]
     rows = x.numel() // cols
     if out is None:

@@ -194,6 +194,9 @@ int ab200_rmsnorm(const void *x, int x_dtype, const void *weight_f16, void *out_
  * position pos[r] (int32 device array); inv_freq fp32 [D/2 or D]. Rotate-half convention. */
 int ab200_rope(const void *x, const float *inv_freq, const int32_t *pos, void *out, int rows,
                int H, int D, int dtype, void *stream);
+/* The same for one row whose position is a host value (the call site's own form). */
+int ab200_rope_at(const void *x, const float *inv_freq, int pos, void *out, int H, int D,
+                  int dtype, void *stream);
 
 /* Row softmax — AntaresIR.md:226.  x, out [rows, cols] in dtype. */
 int ab200_softmax(const void *x, void *out, int rows, int cols, int dtype, void *stream);
@@ -205,6 +208,11 @@ int ab200_softmax(const void *x, void *out, int rows, int cols, int dtype, void 
 int ab200_attention_decode(const void *q, const void *k_cache, const void *v_cache, void *out,
                            const int32_t *seq_len_dev, int seq_len_add, int max_seq, int H, int D,
                            long kv_stride, float scale, int dtype, void *stream);
+/* The same with the number of rows as a host value and att_f read on the device (the call site's own
+ * form: neither needs a copy or a synchronisation). */
+int ab200_attention_decode_at(const void *q, const void *k_cache, const void *v_cache, void *out,
+                              int seq_len, int H, int D, long kv_stride, const float *scale_dev,
+                              int dtype, void *stream);
 
 /* ---- decode-step glue (replaces torch eager ops in samples/05_llama2_7b_int4.py:146-177) -- */
 
