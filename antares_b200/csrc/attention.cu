@@ -8,6 +8,9 @@
 
 namespace ab200 {
 
+int attention_prefill_launch(const void *q, const void *kc, const void *vc, void *out, const int32_t *pos0_dev, int rows, int max_seq, int H, long kv_stride,
+                             float scale, KvPages pages, cudaStream_t stream);  // attention_prefill.cu
+
 constexpr int ATT_THREADS = 256;
 constexpr int ATT_D = 128;
 
@@ -453,6 +456,8 @@ extern "C" int ab200_attention_fused_paged(const void *vqk_f16, const float *inv
   return attention_fused_impl(vqk_f16, inv_freq, pos_dev, k_cache_f16, v_cache_f16, out_f16, H, D, kv_stride, max_seq, scale, page_table, page_rows, stream);
 }
 
+constexpr int ATT_PREFILL_TC_ROWS = 9;
+
 // Causal attention of `rows` consecutive tokens over a cache that already holds their keys and
 // values: query row r (position *pos0_dev + r) attends cache rows 0 .. *pos0_dev + r.  The batched
 // form of ab200_attention_decode (grid = heads x rows).
@@ -467,6 +472,9 @@ static int attention_prefill_impl(const void *q_f16, const void *k_cache_f16, co
   AB200_REQUIRE(aligned16(q_f16) && aligned16(k_cache_f16) && aligned16(v_cache_f16) && aligned16(out_f16), "attention_prefill: pointers must be 16-byte aligned");
   const size_t smem = ((size_t)max_seq + 16 * ATT_D) * sizeof(float);
   if (smem > 200 * 1024) return fail(AB200_EUNSUPPORTED, "attention_prefill: max_seq=%d exceeds the shared-memory score buffer", max_seq);
+  if (rows >= ATT_PREFILL_TC_ROWS)
+    return attention_prefill_launch(q_f16, k_cache_f16, v_cache_f16, out_f16, pos0_dev, rows, max_seq, H, kv_stride, scale,
+                                    KvPages{page_table, page_table ? page_shift_of(page_rows) : 0}, (cudaStream_t)stream);
   if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
   attention_decode_kernel<__half><<<dim3(H, rows), ATT_THREADS, smem, (cudaStream_t)stream>>>(
       (const __half *)q_f16, (const __half *)k_cache_f16, (const __half *)v_cache_f16, (__half *)out_f16, pos0_dev, 1, max_seq, kv_stride, scale, nullptr,
