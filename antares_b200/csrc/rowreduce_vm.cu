@@ -3,103 +3,91 @@
 //   t0[N] >=! f0(x[N, C]);  t1[N] +=! f1(x[N, C], t0[N]);  out[N, C] = g(x[N, C], t0[N], t1[N])
 // (softmax, AntaresIR.md:226; layernorm, AntaresIR.md:232).  The reference compiles each statement
 // into its own generated kernel (lang/einstein_v2.py:297-578 -> antares/default_codegen.py); here one
-// kernel runs all stages of a row back to back: every stage's expression is a small stack program
+// kernel runs all stages of a row back to back: every stage's expression is a small postfix program
 // (the same operation set as the element-wise interpreter, plus "row value of an earlier stage",
-// "column vector" and "number of columns"), evaluated per element in fp32; a reduction stage folds
-// the values of a row with + / max / min (warp shuffles, one shared-memory hop, fixed order, so
-// results are bitwise repeatable), the final stage writes the output.  The row stays in L1/L2
-// between stages, so HBM sees each input once.
+// "column vector" and "number of columns"), run by the accumulator machine of vm_machine.cuh in fp32, eight
+// elements of a thread at a time; a reduction stage folds the values of a row with + / max / min (warp shuffles,
+// one shared-memory hop, fixed order, so results are bitwise repeatable), the final stage writes the output.  The
+// row stays in L1/L2 between stages, so HBM sees each input once.  The block is as wide as the row needs (32 to 256
+// threads), so short rows do not leave warps idle.
 #include <math_constants.h>
 
-#include "common.cuh"
+#include "vm_machine.cuh"
 
 namespace ab200 {
 
-constexpr int RV_MAX_STAGES = 4, RV_MAX_OPS = 48, RV_MAX_CONSTS = 16, RV_MAX_MAT = 4, RV_MAX_COL = 4, RV_MAX_STACK = 8;
-constexpr int RV_THREADS = 256;
+constexpr int RV_MAX_STAGES = 4, RV_MAX_MAT = 4, RV_MAX_COL = 4;
+constexpr int RV_MAX_THREADS = 256;
 
-// operation codes: 0-21 as in the element-wise interpreter (eltwise_vm.cu), then
-enum { RV_IN = 0, RV_CONST = 1, RV_ADD = 2, RV_SUB, RV_MUL, RV_DIV, RV_NEG, RV_EXP, RV_LOG, RV_SQRT, RV_RSQRT, RV_TANH, RV_ERF, RV_SIN, RV_COS,
-       RV_ABS, RV_FLOOR, RV_CEIL, RV_MAX, RV_MIN, RV_POW, RV_SIGMOID, RV_ROW = 22, RV_COL = 23, RV_COLLEN = 24, RV_OP_COUNT };
 enum { RV_MAP = 0, RV_SUM = 1, RV_RMAX = 2, RV_RMIN = 3 };
 
 struct RowProgram {
   const void *mat[RV_MAX_MAT];  // [rows, cols]
   const void *col[RV_MAX_COL];  // [cols]
   void *out;                    // [rows, cols]
-  float cst[RV_MAX_CONSTS];
-  unsigned char op[RV_MAX_STAGES][RV_MAX_OPS], arg[RV_MAX_STAGES][RV_MAX_OPS];
-  unsigned char n_ops[RV_MAX_STAGES], reduce[RV_MAX_STAGES];
+  float cst[VM_MAX_CONSTS];
+  unsigned code[RV_MAX_STAGES][VM_MAX_OPS];
+  VmTemps temps[RV_MAX_STAGES];  // what a stage computes once per row
+  unsigned char n_code[RV_MAX_STAGES], reduce[RV_MAX_STAGES];
   unsigned char mat_f16[RV_MAX_MAT], col_f16[RV_MAX_COL];
-  int n_stages, out_f16, rows, cols;
+  int n_stages, out_f16, rows, cols, vec_ok;
 };
 
-__device__ __forceinline__ float rv_load(const void *p, bool f16, size_t i) {
-  return f16 ? __half2float(reinterpret_cast<const __half *>(p)[i]) : reinterpret_cast<const float *>(p)[i];
-}
-
-__global__ void __launch_bounds__(RV_THREADS) rowreduce_vm_kernel(const __grid_constant__ RowProgram p) {
-  __shared__ float st[RV_MAX_STACK][RV_THREADS];
-  __shared__ float warp_part[RV_THREADS / 32];
-  __shared__ float rowval[RV_MAX_STAGES];
+__global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const __grid_constant__ RowProgram p) {
+  extern __shared__ float4 vm_stack[];
+  // [row parity]: a warp that is a row ahead writes the other half (every row with a reduction has a barrier)
+  __shared__ float part[2][RV_MAX_STAGES][RV_MAX_THREADS / 32];
+  __shared__ unsigned code[RV_MAX_STAGES][VM_MAX_OPS], pre[RV_MAX_STAGES][VM_MAX_OPS];
+  for (int i = threadIdx.x; i < RV_MAX_STAGES * VM_MAX_OPS; i += blockDim.x) {
+    (&code[0][0])[i] = p.code[i / VM_MAX_OPS][i % VM_MAX_OPS];
+    (&pre[0][0])[i] = p.temps[i / VM_MAX_OPS].code[i % VM_MAX_OPS];
+  }
+  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int row = blockIdx.x; row < p.rows; row += gridDim.x) {
+  const unsigned threads = blockDim.x, step = p.vec_ok ? 1 : threads;
+  const int per_pass = (int)threads * VM_E;
+  int parity = 0;
+  for (int row = blockIdx.x; row < p.rows; row += gridDim.x, parity ^= 1) {
     const size_t base = (size_t)row * p.cols;
+    float r0 = 0.f, r1 = 0.f, r2 = 0.f;  // results of the reduction stages
     for (int s = 0; s < p.n_stages; ++s) {
       const int kind = p.reduce[s];
+      float t0 = 0.f, t1 = 0.f, t2 = 0.f, t3 = 0.f;
+      auto scalar = [&](unsigned k, unsigned arg) {
+        return k == VM_K_CONST    ? p.cst[arg]
+               : k == VM_K_COLLEN ? (float)p.cols
+               : k == VM_K_TEMP   ? (arg == 0 ? t0 : arg == 1 ? t1 : arg == 2 ? t2 : t3)
+                                  : (arg == 0 ? r0 : arg == 1 ? r1 : r2);
+      };
+#pragma unroll 1
+      for (int i = 0; i < p.temps[s].n; ++i) {
+        float v[1];
+        const float none[1] = {0.f};
+        vm_run<1>(pre[s] + p.temps[s].start[i], p.temps[s].start[i + 1] - p.temps[s].start[i], vm_stack + threadIdx.x, threads, v, none, scalar,
+                  [](unsigned, unsigned, float(&)[1]) {});
+        if (i == 0) t0 = v[0];
+        else if (i == 1) t1 = v[0];
+        else if (i == 2) t2 = v[0];
+        else t3 = v[0];
+      }
       float acc = kind == RV_RMAX ? -CUDART_INF_F : kind == RV_RMIN ? CUDART_INF_F : 0.f;
-      for (int c = threadIdx.x; c < p.cols; c += RV_THREADS) {
-        // the top of the operand stack stays in a register; shared memory holds what is underneath it
-        int sp = 0;
-        float top = 0.f;
-        for (int k = 0; k < p.n_ops[s]; ++k) {
-          const int op = p.op[s][k], arg = p.arg[s][k];
-          if (op <= RV_CONST || op >= RV_ROW) {
-            if (k > 0) st[sp++][threadIdx.x] = top;
-            if (op == RV_IN) top = rv_load(p.mat[arg], p.mat_f16[arg], base + c);
-            else if (op == RV_CONST) top = p.cst[arg];
-            else if (op == RV_ROW) top = rowval[arg];
-            else if (op == RV_COL) top = rv_load(p.col[arg], p.col_f16[arg], c);
-            else top = (float)p.cols;
-          } else if (op <= RV_DIV || (op >= RV_MAX && op <= RV_POW)) {
-            const float b = top, a = st[--sp][threadIdx.x];
-            switch (op) {
-              case RV_ADD: top = a + b; break;
-              case RV_SUB: top = a - b; break;
-              case RV_MUL: top = a * b; break;
-              case RV_DIV: top = a / b; break;
-              case RV_MAX: top = fmaxf(a, b); break;
-              case RV_MIN: top = fminf(a, b); break;
-              default: top = powf(a, b); break;
-            }
-          } else {
-            const float a = top;
-            switch (op) {
-              case RV_NEG: top = -a; break;
-              case RV_EXP: top = expf(a); break;
-              case RV_LOG: top = logf(a); break;
-              case RV_SQRT: top = sqrtf(a); break;
-              case RV_RSQRT: top = rsqrtf(a); break;
-              case RV_TANH: top = tanhf(a); break;
-              case RV_ERF: top = erff(a); break;
-              case RV_SIN: top = sinf(a); break;
-              case RV_COS: top = cosf(a); break;
-              case RV_ABS: top = fabsf(a); break;
-              case RV_FLOOR: top = floorf(a); break;
-              case RV_CEIL: top = ceilf(a); break;
-              default: top = 1.0f / (1.0f + expf(-a)); break;  // RV_SIGMOID
-            }
-          }
-        }
+      for (int c0 = 0; c0 < p.cols; c0 += per_pass) {
+        const int c = c0 + (int)threadIdx.x * (p.vec_ok ? VM_E : 1);
+        const int left = c < p.cols ? (p.cols - c + (int)step - 1) / (int)step : 0;
+        const int count = left < VM_E ? left : VM_E;
+        const bool vec = p.vec_ok && count == VM_E;
+        float first[VM_E], t[VM_E];
+        vm_load(p.mat[0], p.mat_f16[0], base + c, step, count, vec, first);
+        vm_run<VM_E>(code[s], p.n_code[s], vm_stack + threadIdx.x, threads, t, first, scalar, [&](unsigned k, unsigned arg, float(&b)[VM_E]) {
+          if (k == VM_K_COL) vm_load(p.col[arg], p.col_f16[arg], c, step, count, vec, b);
+          else vm_load(p.mat[arg], p.mat_f16[arg], base + c, step, count, vec, b);
+        });
         if (kind == RV_MAP) {
-          if (p.out_f16) reinterpret_cast<__half *>(p.out)[base + c] = __float2half_rn(top);
-          else reinterpret_cast<float *>(p.out)[base + c] = top;
-        } else if (kind == RV_SUM) {
-          acc += top;
-        } else if (kind == RV_RMAX) {
-          acc = fmaxf(acc, top);
+          vm_store(p.out, p.out_f16, base + c, step, count, vec, t);
         } else {
-          acc = fminf(acc, top);
+#pragma unroll
+          for (int j = 0; j < VM_E; ++j)
+            if (j < count) acc = kind == RV_SUM ? acc + t[j] : kind == RV_RMAX ? fmaxf(acc, t[j]) : fminf(acc, t[j]);
         }
       }
       if (kind != RV_MAP) {
@@ -108,17 +96,18 @@ __global__ void __launch_bounds__(RV_THREADS) rowreduce_vm_kernel(const __grid_c
           const float other = __shfl_xor_sync(0xffffffffu, acc, o);
           acc = kind == RV_SUM ? acc + other : kind == RV_RMAX ? fmaxf(acc, other) : fminf(acc, other);
         }
-        if (lane == 0) warp_part[warp] = acc;
+        if (lane == 0) part[parity][s][warp] = acc;
         __syncthreads();
-        if (threadIdx.x == 0) {
-          float r = warp_part[0];
-          for (int w = 1; w < RV_THREADS / 32; ++w) r = kind == RV_SUM ? r + warp_part[w] : kind == RV_RMAX ? fmaxf(r, warp_part[w]) : fminf(r, warp_part[w]);
-          rowval[s] = r;
+        float r = part[parity][s][0];
+        for (int w = 1; w < (int)threads / 32; ++w) {
+          const float other = part[parity][s][w];
+          r = kind == RV_SUM ? r + other : kind == RV_RMAX ? fmaxf(r, other) : fminf(r, other);
         }
-        __syncthreads();
+        if (s == 0) r0 = r;
+        else if (s == 1) r1 = r;
+        else r2 = r;
       }
     }
-    __syncthreads();  // rowval and warp_part are reused by the next row
   }
 }
 
@@ -133,7 +122,7 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
   clear_error();
   AB200_REQUIRE(ops_host && args_host && stage_len_host && stage_reduce_host && out, "rowreduce_vm: null pointer");
   AB200_REQUIRE(n_stages >= 1 && n_stages <= RV_MAX_STAGES, "rowreduce_vm: %d stages (1..%d)", n_stages, RV_MAX_STAGES);
-  AB200_REQUIRE(n_consts >= 0 && n_consts <= RV_MAX_CONSTS && (n_consts == 0 || consts_host), "rowreduce_vm: %d constants (at most %d)", n_consts, RV_MAX_CONSTS);
+  AB200_REQUIRE(n_consts >= 0 && n_consts <= VM_MAX_CONSTS && (n_consts == 0 || consts_host), "rowreduce_vm: %d constants (at most %d)", n_consts, VM_MAX_CONSTS);
   AB200_REQUIRE(n_mat >= 1 && n_mat <= RV_MAX_MAT && mat_inputs_host && mat_dtypes_host, "rowreduce_vm: %d [rows, cols] inputs (1..%d)", n_mat, RV_MAX_MAT);
   AB200_REQUIRE(n_col >= 0 && n_col <= RV_MAX_COL && (n_col == 0 || (col_inputs_host && col_dtypes_host)), "rowreduce_vm: %d [cols] inputs (at most %d)", n_col, RV_MAX_COL);
   AB200_REQUIRE(rows > 0 && cols > 0, "rowreduce_vm: rows=%d cols=%d", rows, cols);
@@ -151,34 +140,34 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
   }
   for (int i = 0; i < n_consts; ++i) p.cst[i] = consts_host[i];
   // validate every stage on the host: operand indices, stack discipline, stage order
-  int off = 0;
+  int off = 0, stack = 0;
   for (int s = 0; s < n_stages; ++s) {
     const int len = stage_len_host[s], kind = stage_reduce_host[s];
-    AB200_REQUIRE(len >= 1 && len <= RV_MAX_OPS, "rowreduce_vm: stage %d has %d operations (1..%d)", s, len, RV_MAX_OPS);
+    AB200_REQUIRE(len >= 1 && len <= VM_MAX_OPS, "rowreduce_vm: stage %d has %d operations (1..%d)", s, len, VM_MAX_OPS);
     AB200_REQUIRE(kind >= RV_MAP && kind <= RV_RMIN, "rowreduce_vm: stage %d has reduction kind %d", s, kind);
     AB200_REQUIRE((kind == RV_MAP) == (s == n_stages - 1), "rowreduce_vm: the last stage, and only the last, writes the output");
     int depth = 0;
     for (int k = 0; k < len; ++k) {
       const int op = ops_host[off + k], arg = args_host[off + k];
-      AB200_REQUIRE(op < RV_OP_COUNT, "rowreduce_vm: unknown operation %d", op);
-      if (op <= RV_CONST || op >= RV_ROW) {
-        AB200_REQUIRE(op != RV_IN || arg < n_mat, "rowreduce_vm: matrix input index %d out of range", arg);
-        AB200_REQUIRE(op != RV_CONST || arg < n_consts, "rowreduce_vm: constant index %d out of range", arg);
-        AB200_REQUIRE(op != RV_ROW || arg < s, "rowreduce_vm: stage %d reads the row value of stage %d, which is not earlier", s, arg);
-        AB200_REQUIRE(op != RV_COL || arg < n_col, "rowreduce_vm: column-vector index %d out of range", arg);
+      AB200_REQUIRE(op <= VM_COLLEN, "rowreduce_vm: unknown operation %d", op);
+      if (vm_is_leaf(op)) {
+        AB200_REQUIRE(op != VM_IN || arg < n_mat, "rowreduce_vm: matrix input index %d out of range", arg);
+        AB200_REQUIRE(op != VM_CONST || arg < n_consts, "rowreduce_vm: constant index %d out of range", arg);
+        AB200_REQUIRE(op != VM_ROW || arg < s, "rowreduce_vm: stage %d reads the row value of stage %d, which is not earlier", s, arg);
+        AB200_REQUIRE(op != VM_COL || arg < n_col, "rowreduce_vm: column-vector index %d out of range", arg);
         ++depth;
-      } else if (op <= RV_DIV || (op >= RV_MAX && op <= RV_POW)) {
+      } else if (vm_is_binary(op)) {
         AB200_REQUIRE(depth >= 2, "rowreduce_vm: stack underflow in stage %d", s);
         --depth;
       } else {
         AB200_REQUIRE(depth >= 1, "rowreduce_vm: stack underflow in stage %d", s);
       }
-      AB200_REQUIRE(depth <= RV_MAX_STACK, "rowreduce_vm: stage %d needs a stack deeper than %d", s, RV_MAX_STACK);
-      p.op[s][k] = (unsigned char)op;
-      p.arg[s][k] = (unsigned char)arg;
+      AB200_REQUIRE(depth <= VM_MAX_STACK, "rowreduce_vm: stage %d needs a stack deeper than %d", s, VM_MAX_STACK);
     }
     AB200_REQUIRE(depth == 1, "rowreduce_vm: stage %d leaves %d values on the stack", s, depth);
-    p.n_ops[s] = (unsigned char)len;
+    int depth_used = 0;
+    p.n_code[s] = (unsigned char)vm_translate(ops_host + off, args_host + off, len, p.code[s], &depth_used, &p.temps[s]);
+    if (depth_used > stack) stack = depth_used;
     p.reduce[s] = (unsigned char)kind;
     off += len;
   }
@@ -187,8 +176,15 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
   p.out_f16 = out_dtype == AB200_F16;
   p.rows = rows;
   p.cols = cols;
-  const int cap = sm_count() * 8;
-  rowreduce_vm_kernel<<<rows < cap ? rows : cap, RV_THREADS, 0, (cudaStream_t)stream>>>(p);
+  p.vec_ok = cols % VM_E == 0 && aligned16(out);
+  for (int i = 0; i < n_mat; ++i) p.vec_ok = p.vec_ok && aligned16(mat_inputs_host[i]);
+  for (int i = 0; i < n_col; ++i) p.vec_ok = p.vec_ok && aligned16(col_inputs_host[i]);
+  int threads = 32;
+  while (threads < RV_MAX_THREADS && threads * VM_E < cols) threads *= 2;
+  const int cap = sm_count() * (2048 / threads);
+  const size_t smem = (size_t)stack * threads * VM_E * sizeof(float);
+  if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(rowreduce_vm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  rowreduce_vm_kernel<<<rows < cap ? rows : cap, threads, smem, (cudaStream_t)stream>>>(p);
   AB200_CHECK_LAUNCH("rowreduce_vm");
   return AB200_OK;
 }
