@@ -427,33 +427,108 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f16_kernel(GemvParams
 }
 
 // fp32 activations / scales / result: the dtypes the in-tree sample declares
-// (samples/05_llama2_7b_int4.py:75,133,139).  w = scale * (q - 8) is one fp32 multiply, as in
-// IR statement 2; products accumulate in fp32.
+// (samples/05_llama2_7b_int4.py:75,133,139).
+//
+// Raw nibbles again, as fp32 bit patterns: a nibble left at bits 4j (j = 0..5) of a word is the number
+// q * 2^(4j - 149) - a subnormal, and for j = 5, whose top bit is the exponent's lowest, still linear in q - so
+// `w & (15 << 4j)` goes straight into an FFMA with x * 2^(e - 4j); the word shifted right by 8 gives the last two.
+// The powers of two are exact: x is staged once as x * 2^e (2^e from the slice's largest magnitude, so that products
+// stay normal) times 2^(-4j), the zero-point leaves the loop as 8 * sum(x) per 32-k unit and the group scale is applied
+// per unit.  9 logic + 8 FFMA per packed word, against 8 shifts, 8 LOP3, 8 FADD, 8 FMUL, 8 FFMA when every nibble is
+// turned into scale * (q - 8) first.  A chain is the 8 k of one word, so that rounding errors stay below that form's.
+// A slice of x with an infinity or a NaN takes the plain form, whose special values are the operator's.
+// As in the fp16 kernel two units per warp are in flight in registers, the first before griddepcontrol.wait.
 template <int M>
 __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f32_kernel(GemvParams p) {
-  pdl_launch_dependents();
-  pdl_wait();  // this variant has no preamble worth overlapping: wait first
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned cs = cluster.num_blocks(), krank = cluster.block_rank();
-  if (cs > 1) cluster_arrive_started();
   const int tile = blockIdx.x / cs;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n0 = tile * TILE_N + lane * 4;
-  const bool col_ok = n0 < p.N;
+  const int n0 = tile * TILE_N + lane * 4, n0c = n0 < p.N ? n0 : p.N - 4;  // columns beyond N: read the last ones, never stored
   const int u_begin = (int)((long)p.units * krank / cs), u_end = (int)((long)p.units * (krank + 1) / cs);
   const int k_begin = u_begin * UNIT_K, kslice = (u_end - u_begin) * UNIT_K;
+  const int n_units = u_end - u_begin;
 
   const int xs_stride = p.xs_stride;
   float *xs = reinterpret_cast<float *>(smem_raw);
   float *red = xs + (size_t)M * xs_stride;
   float *part = red + GEMV_WARPS * M * TILE_N;
+  float *corr = part + M * TILE_N;  // [M][units of the slice]: 8 * sum over the unit of x
+  __shared__ unsigned sh_max[M][GEMV_WARPS];
 
+  constexpr int NBUF = 2;
+  uint4 wbuf[NBUF][UNIT_ROWS];
+  float4 sbuf[NBUF];
+  int u = u_begin + warp, u_load = u;
+  const int32_t *qcol = p.qw + n0c;
+  const float *scol = reinterpret_cast<const float *>(p.scales) + n0c;
+  auto load_unit = [&](int b) {
+    const int32_t *q = qcol + (size_t)u_load * UNIT_ROWS * p.N;
+#pragma unroll
+    for (int r = 0; r < UNIT_ROWS; ++r) wbuf[b][r] = ldg_stream_v4(q + (size_t)r * p.N);
+    const uint4 sv = ldg_stream_v4(scol + (size_t)((u_load * UNIT_K) / p.group) * p.N);
+    sbuf[b] = make_float4(__uint_as_float(sv.x), __uint_as_float(sv.y), __uint_as_float(sv.z), __uint_as_float(sv.w));
+    u_load += GEMV_WARPS;
+  };
+  if (cs > 1) cluster_arrive_started();
+  pdl_launch_dependents();
+#pragma unroll
+  for (int b = 0; b < NBUF; ++b)
+    if (u_load < u_end) load_unit(b);
+  pdl_wait();  // x (and the output buffer) may come from the kernel before this one
+
+  // stage x; per batch row the largest magnitude of the slice
   const float *xg = reinterpret_cast<const float *>(p.x);
-  for (int i = threadIdx.x; i < M * (kslice / 4); i += GEMV_THREADS) {
-    const int m = i / (kslice / 4), r = i % (kslice / 4);
-    *reinterpret_cast<float4 *>(xs + (size_t)m * xs_stride + r * 4) =
-        *reinterpret_cast<const float4 *>(xg + (size_t)m * p.K + k_begin + r * 4);
+  const int quads = kslice / 4;
+  unsigned mx[M];
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    mx[m] = 0u;
+    for (int i = threadIdx.x; i < quads; i += GEMV_THREADS) {
+      const uint4 v = *reinterpret_cast<const uint4 *>(xg + (size_t)m * p.K + k_begin + i * 4);
+      *reinterpret_cast<uint4 *>(xs + (size_t)m * xs_stride + i * 4) = v;
+      mx[m] = max(mx[m], max(max(v.x & 0x7FFFFFFFu, v.y & 0x7FFFFFFFu), max(v.z & 0x7FFFFFFFu, v.w & 0x7FFFFFFFu)));
+    }
+    mx[m] = __reduce_max_sync(0xffffffffu, mx[m]);
+    if (lane == 0) sh_max[m][warp] = mx[m];
+  }
+  __syncthreads();
+  bool plain = false;
+  float back1[M], back2[M];  // 2^(149 - e) as two factors
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    unsigned t = 0u;
+#pragma unroll
+    for (int w = 0; w < GEMV_WARPS; ++w) t = max(t, sh_max[m][w]);
+    const int E = max((int)(t >> 23), 1);  // biased exponent: |x| < 2^(E - 126)
+    plain = plain || E == 255;
+    // |x| * 2^e < 2^120, products below 15 * 2^-29; e is 246 - E as two exact factors
+    const int e = 246 - E, e1 = e / 2, e2 = e - e1;
+    const float f1 = __int_as_float((127 + e1) << 23), f2 = __int_as_float((127 + e2) << 23);
+    const int b1 = (149 - e) / 2, b2 = 149 - e - b1;
+    back1[m] = __int_as_float((127 + b1) << 23);
+    back2[m] = __int_as_float((127 + b2) << 23);
+    // second pass over the same elements: x * 2^e * 2^(-4j) with j = 0 .. 5, 4, 5 for k = 0 .. 7, and the unit sums
+    // (two quads = one packed row; eight adjacent lanes = one unit)
+    if (E != 255) {
+      const int pad = (quads + 31) & ~31;
+      for (int i = threadIdx.x; i < pad; i += GEMV_THREADS) {
+        float sx = 0.f;
+        if (i < quads) {
+          float4 *slot = reinterpret_cast<float4 *>(xs + (size_t)m * xs_stride + i * 4);
+          const float4 v = *slot;
+          sx = (v.x + v.y) + (v.z + v.w);
+          const float4 w = make_float4(v.x * f1 * f2, v.y * f1 * f2, v.z * f1 * f2, v.w * f1 * f2);
+          *slot = (i & 1) ? make_float4(w.x * 0x1p-16f, w.y * 0x1p-20f, w.z * 0x1p-16f, w.w * 0x1p-20f)
+                          : make_float4(w.x, w.y * 0x1p-4f, w.z * 0x1p-8f, w.w * 0x1p-12f);
+        }
+        sx += __shfl_xor_sync(0xffffffffu, sx, 1);
+        sx += __shfl_xor_sync(0xffffffffu, sx, 2);
+        sx += __shfl_xor_sync(0xffffffffu, sx, 4);
+        if (i < quads && (i & 7) == 0) corr[m * n_units + (i >> 3)] = 8.0f * sx;
+      }
+    }
   }
   __syncthreads();
 
@@ -462,34 +537,69 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f32_kernel(GemvParams
   for (int m = 0; m < M; ++m)
 #pragma unroll
     for (int c = 0; c < 4; ++c) facc[m][c] = 0.f;
-
-  const int32_t *qcol = p.qw + n0;
-  const float *scol = reinterpret_cast<const float *>(p.scales) + n0;
-  for (int u = u_begin + warp; u < u_end && col_ok; u += GEMV_WARPS) {
-    uint4 wv[UNIT_ROWS];
-    const int32_t *q = qcol + (size_t)u * UNIT_ROWS * p.N;
-#pragma unroll
-    for (int r = 0; r < UNIT_ROWS; ++r) wv[r] = ldg_stream_v4(q + (size_t)r * p.N);
-    const float4 s4 = *reinterpret_cast<const float4 *>(scol + (size_t)((u * UNIT_K) / p.group) * p.N);
-    const float sc[4] = {s4.x, s4.y, s4.z, s4.w};
+  auto compute_unit = [&](int b) {
+    const float sc[4] = {sbuf[b].x, sbuf[b].y, sbuf[b].z, sbuf[b].w};
     const float *xu = xs + (u - u_begin) * UNIT_K;
+    if (!plain) {
+      float acc[UNIT_ROWS][M][4];
 #pragma unroll
-    for (int r = 0; r < UNIT_ROWS; ++r) {
-      const uint32_t wr[4] = {wv[r].x, wv[r].y, wv[r].z, wv[r].w};
+      for (int r = 0; r < UNIT_ROWS; ++r) {
+        float4 xa[M], xb[M];
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float xv[M];
-#pragma unroll
-        for (int m = 0; m < M; ++m) xv[m] = xu[(size_t)m * xs_stride + r * 8 + j];
+        for (int m = 0; m < M; ++m) {
+          xa[m] = *reinterpret_cast<const float4 *>(xu + (size_t)m * xs_stride + r * 8);
+          xb[m] = *reinterpret_cast<const float4 *>(xu + (size_t)m * xs_stride + r * 8 + 4);
+        }
+        const uint32_t wr[4] = {wbuf[b][r].x, wbuf[b][r].y, wbuf[b][r].z, wbuf[b][r].w};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          // 2^23 + q as a float, minus (2^23 + 8): q - 8 exactly.
-          const float qm8 = __uint_as_float(0x4B000000u | ((wr[c] >> (4 * j)) & 15u)) - 8388616.0f;
-          const float w = sc[c] * qm8;
+          const uint32_t w = wr[c], w8 = w >> 8;
+          const float q[8] = {__uint_as_float(w & 0xFu),       __uint_as_float(w & 0xF0u),     __uint_as_float(w & 0xF00u),    __uint_as_float(w & 0xF000u),
+                              __uint_as_float(w & 0xF0000u),   __uint_as_float(w & 0xF00000u), __uint_as_float(w8 & 0xF0000u), __uint_as_float(w8 & 0xF00000u)};
 #pragma unroll
-          for (int m = 0; m < M; ++m) facc[m][c] = fmaf(xv[m], w, facc[m][c]);
+          for (int m = 0; m < M; ++m) {
+            float t = q[0] * xa[m].x;
+            t = fmaf(q[1], xa[m].y, t);
+            t = fmaf(q[2], xa[m].z, t);
+            t = fmaf(q[3], xa[m].w, t);
+            t = fmaf(q[4], xb[m].x, t);
+            t = fmaf(q[5], xb[m].y, t);
+            t = fmaf(q[6], xb[m].z, t);
+            acc[r][m][c] = fmaf(q[7], xb[m].w, t);
+          }
         }
       }
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const float zp = corr[m * n_units + (u - u_begin)];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) facc[m][c] = fmaf(sc[c], fmaf(((acc[0][m][c] + acc[1][m][c]) + (acc[2][m][c] + acc[3][m][c])) * back1[m], back2[m], -zp), facc[m][c]);
+      }
+    } else {
+#pragma unroll 1
+      for (int r = 0; r < UNIT_ROWS; ++r) {
+        const uint4 wv = r == 0 ? wbuf[b][0] : r == 1 ? wbuf[b][1] : r == 2 ? wbuf[b][2] : wbuf[b][3];
+        const uint32_t wr[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll 1
+        for (int j = 0; j < 8; ++j) {
+#pragma unroll
+          for (int m = 0; m < M; ++m) {
+            const float xv = xg[(size_t)m * p.K + (size_t)u * UNIT_K + r * 8 + j];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) facc[m][c] = fmaf(xv, sc[c] * (float)((int)((wr[c] >> (4 * j)) & 15u) - 8), facc[m][c]);
+          }
+        }
+      }
+    }
+  };
+  while (u < u_end) {
+#pragma unroll
+    for (int b = 0; b < NBUF; ++b) {
+      if (u < u_end) {
+        compute_unit(b);
+        if (u_load < u_end) load_unit(b);
+      }
+      u += GEMV_WARPS;
     }
   }
   reduce_and_store<M, EPI_STORE_F32, GEMV_THREADS, GEMV_WARPS>(facc, red, part, p.out, p.N, tile * TILE_N);
