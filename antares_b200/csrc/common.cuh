@@ -40,7 +40,7 @@ int *kernel_error_ptr();  // device address of the status word that ab200_kernel
 // the first zero_bytes of it zeroed whenever it is allocated or grown (which also synchronises the device).
 // Callers keep what they need zero between launches themselves.  Not for use under stream capture before
 // the first call; two kernels that use the same buffer must not overlap on the GPU.
-enum { LIB_BUF_PERSIST = 0, LIB_BUF_SLABS, LIB_BUF_TC, LIB_BUF_GEMM, LIB_BUF_COUNT };
+enum { LIB_BUF_PERSIST = 0, LIB_BUF_SLABS, LIB_BUF_TC, LIB_BUF_COUNT };
 int library_buffer(int which, size_t bytes, size_t min_bytes, size_t zero_bytes, void **out);
 
 // Programmatic dependent launch: when enabled (option "pdl"), kernels are launched with

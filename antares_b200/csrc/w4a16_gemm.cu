@@ -1,445 +1,532 @@
-// W4A16 prefill GEMM on the 5th-generation tensor cores: out[M,N] = x[M,K] . dequant(qweight, scales)
-// with fp16 x / scales / out and fp32 accumulation in tensor memory.
+// W4A16 GEMM on the 5th-generation tensor cores: out[M,N] = x[M,K] . dequant(qweight, scales), fp16 in and out, fp32
+// accumulation in tensor memory; and the same with SwiGLU on the way out (weights gate | up, out[M, N/2]).
 //
-// Replaces the exported op of samples/05_llama2_7b_int4.py:135-144 when it is called with a leading
-// M axis larger than the decode path handles.  The dequantised weight fed to the tensor cores is
-// exactly w = RN_fp16(scale * fp16(q - 8)) (IR statement 2), the products accumulate in fp32.
+// Replaces the exported op of samples/05_llama2_7b_int4.py:135-144 for batches above the decode path (and the two
+// projections and silu(gate) * up of :168-172 for a prompt); the weight fed to the tensor cores is
+// w = RN_fp16(scale * fp16(q - 8)) (IR statement 2), the products accumulate in fp32.
 //
-// CTA tile 256 (M) x 256 (N), K step 64, three shared-memory stages, 512 + 96 threads, one CTA per SM.
-// The two 128-row halves of the tile have their own fp32 accumulator (2 x 256 TMEM columns) and
-// share every dequantised weight tile, which halves the dequantisation work per flop against a
-// 128-row tile.  All 512 threads fill a stage:
-//   A: the x tile arrives by TMA (`cp.async.bulk.tensor.2d`, one box of 64 k x 128 rows per
-//      accumulator half, 128-byte swizzle, completion on the stage's mbarrier): whole 128-byte lines
-//      from L2, no thread instructions, and the K-major 128B-swizzled layout the MMA reads natively;
-//   B: thread t owns column n0 + t % 256 and four of the stage's eight packed rows: each packed
-//      int32 word (8 consecutive k of one column) becomes one 16-byte row of a K-major no-swizzle
-//      core matrix (LOP3 + 0x6400 magic, HSUB2/HFMA2 for the zero-point, HMUL2 by the group scale,
-//      PRMT back to natural k order), so no transpose is needed and a quarter-warp writes 128
-//      contiguous bytes.
-// Per stage eight `tcgen05.mma.cta_group::1.kind::f16` (M128 N256 K16, both operands K-major; four K steps
-// x two accumulators) are issued and committed to the stage's mbarrier; a stage is refilled once the MMAs
-// that read it three iterations ago have completed, so filling overlaps the MMAs of the two stages before.
-// Issuing is not free for the issuing thread (descriptors pass through uniform registers, every wait and
-// commit is a dependent instruction): with one thread doing everything a k tile cost that thread more
-// cycles than the tensor pipe needs for its eight MMAs.  So three single-thread roles live in warps 16-18:
-// the MMAs of accumulator 0, the MMAs of accumulator 1 (each commits on its own; the barriers count two
-// arrivals), and the TMA copies of x, which run up to four k tiles ahead.  Producers and issuers meet only
-// through mbarriers (weights ready, x tile landed, MMAs done), there is no block-wide barrier inside the
-// K loop.  The epilogue reads the accumulators with `tcgen05.ld` (row = TMEM lane; the four warps that
-// share a lane quarter split the 512 columns), rounds to fp16 and stores.
-// Short prompts: an accumulator whose 128 rows all lie beyond M is left out (its issuing thread only keeps
-// the barriers in step), and when the problem has fewer tiles than half the SMs the grid's z dimension
-// splits K into up to four ranges: every CTA stores its fp32 accumulators as partial sums (laid out so
-// that a warp's 32 rows of 16 columns are consecutive), the last CTA of a tile to arrive adds the parts in
-// part order - bitwise repeatable - and runs the epilogue.
-// Every mbarrier wait is bounded and reports through the status word.
+// The weights take the M side of the MMA and the rows of x its N side: out^T[n, m] = sum_k w[k, n] x[m, k], M128 N<mt> K16
+// with mt = the rows of a tile rounded up to 16, at most 256.  So the row tile follows the prompt (40 rows cost an MMA of
+// N = 48, not a padded 128) and a weight is dequantised once per 256 rows.  A CTA takes two runs of 128 columns (two
+// accumulators that share the x tile; neighbours, or the gate and up columns of the same 128 outputs) and a range of K in
+// units of 64:
+//   x        `cp.async.bulk.tensor.2d`, 64 k x mt rows, 128-byte swizzle, the K-major operand as it lands
+//   weights  packed words (8 rows x 128 columns, twice) and the group's scales by TMA into their own deeper ring, so that
+//            the HBM stream is not bound to registers.
+// Where the dequantised weights go is the choice between two forms (the host's cost model takes it):
+//   tensor memory (mt <= 192): a thread takes one column of a unit (8 words), turns it into 64 values in k order and stores
+//            them with `tcgen05.st`; the MMA takes its A operand from there.  Accumulators 2 x mt columns, the rest two to
+//            four stages of 2 x 32 columns.
+//   shared memory (mt up to 256, when a round of wide tiles fits the SMs better): a thread takes one packed row of 8
+//            columns, pairs the halves of neighbouring columns (`prmt`) and so gets (column, column + 1) pairs for each of
+//            the 8 k: the operand is written MN-major (a 128-byte row = 64 columns of one k, 128-byte swizzle, no bank
+//            conflicts), without reordering k; three stages of 32 KiB.
+// What bounds them: with weights and x both in shared memory a unit moves 3 mt + 700 cycles' worth of it (128 bytes a
+// cycle) for 4 mt cycles of MMA; with the weights in tensor memory it is the eight MMAs of a unit, which take 85 to 100
+// cycles each however small mt is, 650 + 2 mt a unit in all.  Measured, us, K 4096 N 12288 / 22016: 128 rows 22 / 33, and
+// 48 / 37 with the weights in shared memory; 2048 rows, both forms in play, 163-167 / 290-298.  The kernel before this one
+// (x as the M operand padded to 128, K split through global scratch): 43 / 43 and 170 / 290.
+// Roles: 2 x 8 dequantising warps (units alternate between the two halves), one thread each for the x copies and the
+// packed copies, one warp for the MMAs; they meet through mbarriers.
+// K split: the parts of a tile are the CTAs of one thread-block cluster (at most 8).  After the last MMA every CTA
+// pushes its accumulators, 16 rows of x at a time, as fp32 into their owners' shared memory (distributed shared memory,
+// 512 contiguous bytes per warp and store), and after one cluster barrier each CTA adds its own in rank order (bitwise
+// repeatable).  The library owns no scratch for it: a recorded graph holds no pointer that a later call could move.
+// Every mbarrier wait is bounded and reports through the status word (site 210).
+#include <atomic>
+
+#include <cooperative_groups.h>
 #include <cuda.h>  // CUtensorMap and its enums (types only)
 
 #include "common.cuh"
 
+namespace cg = cooperative_groups;
+
 namespace ab200 {
 
-constexpr int GM_BM = 256, GM_BN = 256, GM_BK = 64;
-constexpr int GM_HM = 128;                     // rows per accumulator (one MMA's M)
-constexpr int GM_FILL_THREADS = 512;               // 16 warps dequantise weights
-constexpr int GM_THREADS = GM_FILL_THREADS + 96;   // + three warps whose lane 0 issues: the MMAs of accumulator 0, of accumulator 1, the TMA copies
-constexpr int GM_STAGES = 3;    // stages of dequantised weights
-constexpr int GM_ASTAGES = 4;   // stages of the x tile: one more, so that its TMA copy is issued two k tiles ahead
-constexpr int GM_AH_BYTES = GM_HM * GM_BK * 2;  // 16 KiB: one 128-row half of the x tile (128 rows x 128 B)
-constexpr int GM_A_BYTES = 2 * GM_AH_BYTES;    // 32 KiB
-constexpr int GM_B_BYTES = GM_BN * GM_BK * 2;  // 32 KiB
-constexpr unsigned GM_WAIT_POLLS = 1u << 22;
+constexpr int GS_BN = 256, GS_BK = 64, GS_MAX_MT = 256, GS_TMEM_MT = 192, GS_MAX_PARTS = 8;
+constexpr int GS_DQ_WARPS = 16;                              // two groups of 8
+constexpr int GS_X_WARP = 16, GS_MMA_WARP = 17, GS_P_WARP = 18;
+constexpr int GS_THREADS = 19 * 32;
+constexpr int GS_DQ_THREADS = GS_DQ_WARPS * 32;
+constexpr int GS_W_COLS = 64;                                // a dequantised unit in tensor memory: 2 x 32 columns
+constexpr int GS_PH_BYTES = (GS_BK / 8) * 128 * 4;            // packed words of one accumulator's columns
+constexpr int GS_P_BYTES = 2 * GS_PH_BYTES + GS_BN * 2;       // packed unit + scales: 8704
+constexpr int GS_W_BYTES = GS_BN * GS_BK * 2;                // the same in shared memory: 2 x [2 blocks of 64 columns][64 k][128 B]
+constexpr int GS_MAX_DX = 6, GS_MAX_DW = 4, GS_MAX_DP = 12;  // ring depths: x, dequantised weights, packed weights (the deepest)
+constexpr int GS_UNIT_BARS = 8;                              // more than any ring of x or weights is deep
+constexpr int GS_ITEM_BYTES = 2 * 128 * 16 * 4;               // K split: 256 columns x 16 rows of x, fp32
+constexpr int GS_ROWB = GS_BN * 2 + 16;                       // bytes per parked output row
+constexpr int GS_SMEM_LIMIT = 227 * 1024 - 1024;             // 1 KiB for the static part
+constexpr int GS_TILE_CYCLES = 6000, GS_SPLIT_CYCLES = 3000, GS_SPLIT_ROW_CYCLES = 30;  // see gemm_launch
+constexpr unsigned GS_WAIT_POLLS = 1u << 22;
 
 struct GemmParams {
-  const __half *x;
-  const int32_t *qw;
-  const __half *scales;
   __half *out;
   int M, K, N, group;
+  int mt;      // rows of x per tile, a multiple of 16
+  int second;  // columns from an accumulator's run of 128 to the other's: 128, or N / 2 (gate | up)
+  int n_out;   // columns of out
+  int dx, dw, dp;  // ring depths
   int *status;
-  int parts;           // K ranges per tile: > 1 when there are too few tiles to fill the GPU
-  float *partial;      // [tiles][parts][16 column chunks][256 rows][16] fp32: K-split partial accumulators
-  unsigned *counters;  // [tiles], zero between launches
 };
 
-__device__ __forceinline__ uint32_t gm_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Shared-memory matrix descriptor, K-major, no swizzle: core matrices of 8 rows x 16 bytes;
-// LBO = bytes between the two 16-byte K chunks of one MMA, SBO = bytes between 8-row groups.
-__device__ __forceinline__ uint64_t gm_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)((lbo_bytes >> 4) & 0x3FFF) << 16;
-  d |= (uint64_t)((sbo_bytes >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;  // descriptor version for sm_100
-  return d;                // base offset 0, layout type 0 (no swizzle)
+__device__ __forceinline__ uint32_t gs_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// 128-byte-swizzled operand: atoms of 8 x 128 B, 1024 B apart; lead: bytes between blocks of 64 elements along MN of an
+// MN-major operand (not used by a K-major one)
+__device__ __forceinline__ uint64_t gs_desc(uint32_t addr, uint32_t lead) {
+  return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((lead >> 4) & 0x3FFF) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
 }
-
-// K-major operand in the 128-byte-swizzled layout TMA writes (rows of 128 B, 8-row atoms of 1024 B):
-// stride between atoms 1024 B, leading-dimension field unused (1), layout type 2 = SWIZZLE_128B.
-__device__ __forceinline__ uint64_t gm_desc_sw128(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-
-__device__ __forceinline__ bool gm_mbar_wait(uint64_t *bar, unsigned parity) {
-  const uint32_t addr = gm_smem_u32(bar);
+__device__ __forceinline__ bool gs_wait(uint32_t bar, unsigned parity) {
   {  // non-blocking probe first: cheaper than try_wait when the phase completed long ago
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done)
-        : "r"(addr), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     if (done) return true;
   }
-  for (unsigned i = 0; i < GM_WAIT_POLLS; ++i) {
+  for (unsigned i = 0; i < GS_WAIT_POLLS; ++i) {
     uint32_t done;
     asm volatile(
         "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(done)
-        : "r"(addr), "r"(parity)
+        : "r"(bar), "r"(parity)
         : "memory");
     if (done) return true;
   }
   return false;
 }
+__device__ __forceinline__ void gs_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void gs_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void gs_tma(uint32_t dst, const CUtensorMap *tm, int x, int y, uint32_t bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
+               "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void gs_commit(uint32_t bar) {  // by the thread that issues the MMAs
+  asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool gs_elect() {
+  uint32_t e;
+  asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(e));
+  return e != 0;
+}
+__device__ __forceinline__ void gs_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+        "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
 
-// SPLIT: the grid's z dimension splits K (few tiles); the unsplit instantiation carries none of that code.
-template <bool SPLIT>
-__global__ void __launch_bounds__(GM_THREADS) w4a16_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x, GemmParams p) {
-  extern __shared__ __align__(1024) unsigned char gm_smem_raw[];
-  unsigned char *gm_smem = gm_smem_raw + ((1024u - (gm_smem_u32(gm_smem_raw) & 1023u)) & 1023u);  // swizzle atoms need 1024-B alignment
-  __shared__ __align__(8) uint64_t mma_bar[GM_STAGES], b_full_bar[GM_STAGES], full_bar[GM_ASTAGES], a_free_bar[GM_ASTAGES];
-  __shared__ uint32_t tmem_base_s;
-  __shared__ int fail_s, last_s;
+__device__ __forceinline__ void gs_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15};" ::"r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]),
+               "r"(r[15]), "r"(taddr)
+               : "memory");
+}
+
+__device__ __forceinline__ float gs_silu_mul(float g, float u) {  // of the fp16 results, as the separate kernel has them
+  g = __half2float(__float2half_rn(g));
+  return g / (1.0f + expf(-g)) * __half2float(__float2half_rn(u));
+}
+
+// SILU: the accumulators are gate and up of the same outputs, out = silu(gate) * up.  TMEM: where the dequantised weights are.
+template <bool SILU, bool TMEM>
+__global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w,
+                                                                         const __grid_constant__ CUtensorMap tm_s, GemmParams p) {
+  extern __shared__ unsigned char gs_raw[];
+  unsigned char *smem = gs_raw + ((1024u - (gs_smem_u32(gs_raw) & 1023u)) & 1023u);  // swizzle atoms need 1024-byte alignment
+  // barriers of unit u (slot u % 8): operands there (eight dequantising warps and the x copy), MMAs complete; of the packed
+  // ring: full, empty [12]; all MMAs complete
+  __shared__ __align__(8) uint64_t bars[2 * GS_UNIT_BARS + 2 * GS_MAX_DP + 1];
+  __shared__ uint32_t tmem_s;
+  __shared__ int fail_s;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int parts = (int)cluster.num_blocks(), part = (int)cluster.block_rank();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m0 = blockIdx.y * GM_BM, n0 = blockIdx.x * GM_BN;
-  const int K = p.K, N = p.N, M = p.M;
-  // K range of this CTA, in k tiles of 64: [kt0, kt0 + ktiles)
-  const int kt0 = SPLIT ? (K / GM_BK) * (int)blockIdx.z / p.parts : 0;
-  const int ktiles = SPLIT ? (K / GM_BK) * ((int)blockIdx.z + 1) / p.parts - kt0 : K / GM_BK;
+  const int n0 = ((int)blockIdx.x / parts) * (SILU ? GS_BN / 2 : GS_BN), mt = p.mt, m0 = (int)blockIdx.y * mt;
+  const int units = p.K / GS_BK, u0 = (int)((long)units * part / parts), n_units = (int)((long)units * (part + 1) / parts) - u0;
+  const int dx = p.dx, dw = p.dw, dp = p.dp;
+  const uint32_t xb = (uint32_t)mt * (GS_BK * 2);
+  const uint32_t b_full = gs_smem_u32(bars), b_used = b_full + 8 * GS_UNIT_BARS, b_pfull = b_used + 8 * GS_UNIT_BARS, b_pempty = b_pfull + 8 * GS_MAX_DP,
+                 b_done = b_pempty + 8 * GS_MAX_DP;
+  auto bar_of = [](uint32_t first, int u) { return first + 8 * (u & (GS_UNIT_BARS - 1)); };
+  auto phase_of = [](int u) { return (unsigned)(u / GS_UNIT_BARS) & 1u; };
+  const uint32_t s_w = gs_smem_u32(smem), s_x = s_w + (TMEM ? 0 : dw * GS_W_BYTES), s_p = s_x + dx * xb;
 
   if (tid == 0) {
-    for (int s = 0; s < GM_STAGES; ++s)
-    {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(gm_smem_u32(&mma_bar[s])));  // one commit per issuing thread
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(gm_smem_u32(&b_full_bar[s])), "r"(GM_FILL_THREADS / 32));
-    }
-    for (int s = 0; s < GM_ASTAGES; ++s) {
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(gm_smem_u32(&full_bar[s])));
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 2;" ::"r"(gm_smem_u32(&a_free_bar[s])));
-    }
+    auto init = [](uint32_t bar, int count) { asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count)); };
+    for (int i = 0; i < GS_UNIT_BARS; ++i) init(b_full + 8 * i, GS_DQ_WARPS / 2 + 1), init(b_used + 8 * i, 1);
+    for (int i = 0; i < GS_MAX_DP; ++i) init(b_pfull + 8 * i, 1), init(b_pempty + 8 * i, GS_DQ_WARPS / 2);
+    init(b_done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fail_s = 0;
   }
-  if (warp == 0) {  // one warp allocates both accumulators: all 512 TMEM columns
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gm_smem_u32(&tmem_base_s)), "r"(2 * GM_BN) : "memory");
+  if (warp == GS_MMA_WARP) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gs_smem_u32(&tmem_s)), "n"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  pdl_launch_dependents();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_acc = tmem_base_s;
+  const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_s, 0), acc1 = (mt + 31) & ~31, tmem_w = tmem + 2 * acc1;  // accumulators, then the weights
+  bool good = true;
 
-  // instruction descriptor: D fp32, A/B fp16, both K-major, N = 256, M = 128
-  constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(GM_BN >> 3) << 17) | ((uint32_t)(GM_HM >> 4) << 24);
-
-  // ---- per-thread fill roles ---------------------------------------------------------------------------
-  // B: column n0 + tid % 256, packed rows bh*4 .. bh*4+3 of the stage's eight.  A column beyond N reads
-  // the last column instead: its accumulator columns are never stored.
-  const int bcol = tid & (GM_BN - 1), bh = tid >> 8;
-  const int nb = min(n0 + bcol, N - 1);
-  const int tiles_per_group = p.group / GM_BK;
-  const int32_t *qptr = p.qw + nb + (size_t)(kt0 * 8 + bh * 4) * N;  // the packed words of the next k tile to load
-  const __half *sptr = p.scales + nb + (size_t)(kt0 / tiles_per_group) * N;  // its scale
-  int group_count = kt0 % tiles_per_group;
-  const uint32_t b_off = (uint32_t)((bcol >> 3) * 128 + (bcol & 7) * 16 + bh * 4 * (GM_BN / 8) * 128);  // + j * 4096
-  // A: thread 0 asks the TMA unit for the two 64 k x 128 row boxes of k tile kt
-  auto issue_a = [&](int kt) {
-    const int s = kt % GM_ASTAGES;
-    const uint32_t bar = gm_smem_u32(&full_bar[s]);
-    const uint32_t dst = gm_smem_u32(gm_smem + s * GM_A_BYTES);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(GM_A_BYTES) : "memory");
-#pragma unroll
-    for (int hm = 0; hm < 2; ++hm)
-      asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst + hm * GM_AH_BYTES),
-                   "l"(reinterpret_cast<uint64_t>(&tm_x)), "r"((kt0 + kt) * GM_BK), "r"(m0 + hm * GM_HM), "r"(bar)
-                   : "memory");
-  };
-
-  // Three register sets for the packed weights: the global loads of k tile kt+3 are issued while
-  // tile kt is being written to shared memory.  Loads are issued in k order, so one running pointer
-  // (and a counter for the scale row) serves all three sets.
-  struct FillRegs {
-    uint32_t b[4];
-    __half s;
-  };
-  auto load_next = [&](FillRegs &r) {  // global -> registers for the next k tile
-    const int32_t *p0 = qptr, *p1 = p0 + N, *p2 = p1 + N, *p3 = p2 + N;
-    // volatile asm: the loads must be ISSUED here, three tiles ahead of their use, not sunk to it
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r.b[0]) : "l"(p0));
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r.b[1]) : "l"(p1));
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r.b[2]) : "l"(p2));
-    asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(r.b[3]) : "l"(p3));
-    unsigned short sbits;
-    asm volatile("ld.global.nc.b16 %0, [%1];" : "=h"(sbits) : "l"(sptr));
-    r.s = __ushort_as_half(sbits);
-    qptr = p3 + (size_t)5 * N;  // eight packed rows on
-    if (++group_count == tiles_per_group) {
-      group_count = 0;
-      sptr += N;
-    }
-  };
-
-  bool ok = true;
-  // Producer warps (0-15): per k tile wait until the MMAs that read the stage three tiles ago are
-  // done, write the dequantised weights, make them visible to the tensor core and arrive (one
-  // arrive per warp) on the stage's "weights ready" barrier.  No block-wide barrier in the loop:
-  // warps drift apart and hide each other's latencies.  `round` = kt / 3; the stage is the call site's.
-  auto fill_step = [&](int stage, int round, bool more, FillRegs &r) {
-    unsigned char *sb = gm_smem + GM_ASTAGES * GM_A_BYTES + stage * GM_B_BYTES;
-    if (round > 0) {
-      if (!gm_mbar_wait(&mma_bar[stage], (round - 1) & 1)) {
-        ok = false;
-        fail_s = 1;
+  if (warp == GS_P_WARP) {
+    if (gs_elect()) {  // packed words and scales
+      for (int u = 0, slot = 0, ph = 1; u < n_units; ++u) {
+        if (u >= dp && !gs_wait(b_pempty + 8 * slot, ph)) {
+          good = false;
+          break;
+        }
+        const uint32_t bar = b_pfull + 8 * slot, dst = s_p + slot * GS_P_BYTES;
+        gs_expect(bar, GS_P_BYTES);
+        const int row = (u0 + u) * (GS_BK / 8), srow = row * 8 / p.group;
+        gs_tma(dst, &tm_w, n0, row, bar);
+        gs_tma(dst + GS_PH_BYTES, &tm_w, n0 + p.second, row, bar);
+        gs_tma(dst + 2 * GS_PH_BYTES, &tm_s, n0, srow, bar);
+        gs_tma(dst + 2 * GS_PH_BYTES + 256, &tm_s, n0 + p.second, srow, bar);
+        if (++slot == dp) slot = 0, ph ^= 1;
       }
+      if (!good) fail_s = 1;
     }
-    {
-      constexpr uint32_t LO = 0x000F000Fu, HI = 0x00F000F0u, MAGIC = 0x64006400u;
-      const __half2 c1032 = u2h2(0x64086408u), c16th = u2h2(0x2C002C00u), cm72 = u2h2(0xD480D480u);
-      const __half2 sc2 = __half2half2(r.s);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint32_t w = r.b[j], w8 = w >> 8;
-        uint4 o;  // (k0,k4)(k1,k5)(k2,k6)(k3,k7), each RN_fp16(scale * (q - 8))
-        o.x = h22u(__hmul2(__hsub2(u2h2(lop3<0xEA>(w, LO, MAGIC)), c1032), sc2));
-        o.y = h22u(__hmul2(__hfma2(u2h2(lop3<0xEA>(w, HI, MAGIC)), c16th, cm72), sc2));
-        o.z = h22u(__hmul2(__hsub2(u2h2(lop3<0xEA>(w8, LO, MAGIC)), c1032), sc2));
-        o.w = h22u(__hmul2(__hfma2(u2h2(lop3<0xEA>(w8, HI, MAGIC)), c16th, cm72), sc2));
-        uint4 n;  // back to natural k order: (k0,k1)(k2,k3)(k4,k5)(k6,k7)
-        n.x = __byte_perm(o.x, o.y, 0x5410);
-        n.y = __byte_perm(o.z, o.w, 0x5410);
-        n.z = __byte_perm(o.x, o.y, 0x7632);
-        n.w = __byte_perm(o.z, o.w, 0x7632);
-        *reinterpret_cast<uint4 *>(sb + j * (GM_BN / 8) * 128 + b_off) = n;
-      }
-    }
-    if (more) load_next(r);  // this set's next tile: three MMA periods to arrive
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
     __syncwarp();
-    if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gm_smem_u32(&b_full_bar[stage])) : "memory");
-  };
-  // Issuers (lane 0 of warps 16 and 17, one per accumulator): the MMAs of a k tile as soon as its weights
-  // and its x tile are in shared memory.  Issuing costs the thread tens of cycles per instruction
-  // (descriptors through uniform registers, waits, commits), so the work is split over two threads
-  // and the TMA copies have a thread of their own.
-  auto issue_mmas = [&](int kt, int hm) {
-    const int s = kt % GM_STAGES, sA = kt % GM_ASTAGES;
-    if (!gm_mbar_wait(&b_full_bar[s], (kt / GM_STAGES) & 1) || !gm_mbar_wait(&full_bar[sA], (kt / GM_ASTAGES) & 1)) {
-      ok = false;
-      fail_s = 1;
+  } else if (warp == GS_X_WARP) {
+    if (gs_elect()) {  // x tiles
+      pdl_wait();      // x comes from the kernel before this one; weights and scales are constant and already on their way
+      for (int u = 0, slot = 0; u < n_units; ++u) {
+        if (u >= dx && !gs_wait(bar_of(b_used, u - dx), phase_of(u - dx))) {
+          good = false;
+          break;
+        }
+        gs_expect(bar_of(b_full, u), xb);
+        gs_tma(s_x + slot * xb, &tm_x, (u0 + u) * GS_BK, m0, bar_of(b_full, u));
+        if (++slot == dx) slot = 0;
+      }
+      if (!good) fail_s = 1;
     }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint64_t da0 = gm_desc_sw128(gm_smem_u32(gm_smem + sA * GM_A_BYTES) + hm * GM_AH_BYTES);
-    const uint64_t db0 = gm_desc(gm_smem_u32(gm_smem + GM_ASTAGES * GM_A_BYTES + s * GM_B_BYTES), (GM_BN / 8) * 128, 128);
-    const uint32_t acc = tmem_acc + hm * GM_BN;
+    __syncwarp();
+  } else if (warp == GS_MMA_WARP) {
+    // The whole warp runs the loop and only the MMAs and commits are one thread's: in a divergent branch every descriptor
+    // would have to be moved into uniform registers on its own.
+    // Instruction descriptor: D fp32, A/B fp16, B K-major, A K-major or (bit 15) MN-major, N = mt, M = 128
+    const uint32_t idesc = (1u << 4) | (TMEM ? 0u : 1u << 15) | ((uint32_t)(mt >> 3) << 17) | (128u >> 4 << 24);
+    // One wait and one commit per unit: at some hundred cycles each they, not the MMAs, are what this loop takes.
+    for (int u = 0, xs = 0, ws = 0; u < n_units; ++u) {
+      good = __all_sync(0xffffffffu, gs_wait(bar_of(b_full, u), phase_of(u)));
+      if (!good) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t b0 = gs_desc(s_x + xs * xb, 16);
 #pragma unroll
-    for (int kb = 0; kb < GM_BK / 16; ++kb) {
-      // 16 k further: 32 B into the swizzled x row, two 16-byte chunks of (BN/8)*128 B into the weight tile
-      const uint64_t da = da0 + (uint64_t)(kb * 2), db = db0 + (uint64_t)(kb * (2 * (GM_BN / 8) * 128 / 16));
-      if (kb == 0) {
-        const uint32_t accumulate = kt > 0 ? 1u : 0u;
-        asm volatile(
-            "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n}\n" ::"r"(acc),
-            "l"(da), "l"(db), "r"(IDESC), "r"(accumulate), "r"(0u)
-            : "memory");
+      for (int k = 0; k < GS_BK / 16; ++k)
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {  // 16 k further: 32 B inside a row of x; 8 columns of tensor memory or two atoms of the weights
+          const uint32_t accumulate = (u > 0 || k > 0) ? 1u : 0u;
+          if constexpr (TMEM)
+            asm volatile(
+                "{\n .reg .pred p, q;\n elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n" ::"r"(
+                    tmem + a * acc1),
+                "r"(tmem_w + ws * GS_W_COLS + a * 32 + k * 8), "l"(b0 + (uint64_t)(k * 2)), "r"(idesc), "r"(accumulate)
+                : "memory");
+          else
+            asm volatile(
+                "{\n .reg .pred p, q;\n elect.sync _|q, 0xffffffff;\n setp.ne.b32 p, %4, 0;\n @q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+                    tmem + a * acc1),
+                "l"(gs_desc(s_w + ws * GS_W_BYTES, GS_BK * 128) + (uint64_t)((a * (GS_W_BYTES / 2) + k * 2048) >> 4)), "l"(b0 + (uint64_t)(k * 2)), "r"(idesc), "r"(accumulate)
+                : "memory");
+        }
+      gs_commit(bar_of(b_used, u));
+      if (++xs == dx) xs = 0;
+      if (++ws == dw) ws = 0;
+    }
+    gs_commit(b_done);
+    if (!good) fail_s = 1;
+  } else {
+    // ---- dequantise: half h takes units h, h + 2, ..
+    // TMEM: a thread has one column, tensor-memory lane q * 32 + lane of accumulator a.
+    // Otherwise: warp r of a half packed row r, lane c columns 8c .. 8c + 7.
+    const int h = warp >> 3, a = TMEM ? (warp >> 2) & 1 : lane >> 4, q = warp & 3, r8 = warp & 7;
+    const unsigned char *ring = smem + (s_p - s_w);
+    const unsigned char *words = ring + a * GS_PH_BYTES + (TMEM ? (q * 32 + lane) * 4 : r8 * 512 + (lane & 15) * 32);
+    const unsigned char *scale = ring + 2 * GS_PH_BYTES + (TMEM ? a * 256 + (q * 32 + lane) * 2 : lane * 16);
+    constexpr uint32_t LO = 0x000F000Fu, HI = 0x00F000F0u, MAGIC = 0x64006400u;
+    const __half2 c1032 = u2h2(0x64086408u), c16th = u2h2(0x2C002C00u), cm72 = u2h2(0xD480D480u);
+    // RN(scale * (q - 8)) of the nibbles at bits 0 and 16 (l0), 4 and 20 (l1), 8 and 24 (l2), 12 and 28 (l3)
+    auto dequant = [&](uint32_t v, __half2 sc, uint32_t &l0, uint32_t &l1, uint32_t &l2, uint32_t &l3) {
+      const uint32_t v8 = v >> 8;
+      l0 = h22u(__hmul2(__hsub2(u2h2(lop3<0xEA>(v, LO, MAGIC)), c1032), sc));
+      l1 = h22u(__hmul2(__hfma2(u2h2(lop3<0xEA>(v, HI, MAGIC)), c16th, cm72), sc));
+      l2 = h22u(__hmul2(__hsub2(u2h2(lop3<0xEA>(v8, LO, MAGIC)), c1032), sc));
+      l3 = h22u(__hmul2(__hfma2(u2h2(lop3<0xEA>(v8, HI, MAGIC)), c16th, cm72), sc));
+    };
+    int ps = h, ws = h, pph = 0;  // ring slots of unit u, kept by counting: no divisions in the loop
+    for (int u = h; u < n_units; u += 2) {
+      // The stage first: once the MMAs of unit u - dw are complete, so is every packed unit up to there, and the packed
+      // ring (at least as deep) cannot be two phases behind what this half, which sees every second unit, waits for.  (Nor
+      // can the barrier waited on here: the MMAs of unit u - 2 - dw are known to be complete.)
+      if (u >= dw) good = __all_sync(0xffffffffu, gs_wait(bar_of(b_used, u - dw), phase_of(u - dw)));
+      good = good && __all_sync(0xffffffffu, gs_wait(b_pfull + 8 * ps, pph));
+      if (!good) break;
+      uint32_t w[8];
+      uint4 sv = make_uint4(0, 0, 0, 0);
+      if constexpr (TMEM) {
+#pragma unroll
+        for (int r = 0; r < 8; ++r) w[r] = *reinterpret_cast<const uint32_t *>(words + ps * GS_P_BYTES + r * 512);
+        sv.x = h22u(__half2half2(*reinterpret_cast<const __half *>(scale + ps * GS_P_BYTES)));
       } else {
-        asm volatile(
-            "{\n .reg .pred p;\n setp.eq.u32 p, 0, 0;\n"
-            " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%4, %4, %4, %4}, p;\n}\n" ::"r"(acc),
-            "l"(da), "l"(db), "r"(IDESC), "r"(0u)
-            : "memory");
-      }
-    }
-    // arrive on the barriers when every MMA this thread issued so far has completed
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gm_smem_u32(&mma_bar[s])) : "memory");
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(gm_smem_u32(&a_free_bar[sA])) : "memory");
-  };
-  if (warp < GM_FILL_THREADS / 32) {
-    FillRegs r0, r1, r2;
-    load_next(r0);
-    if (ktiles > 1) load_next(r1);
-    if (ktiles > 2) load_next(r2);
-    for (int kt = 0, round = 0; kt < ktiles; kt += 3, ++round) {
-      fill_step(0, round, kt + 3 < ktiles, r0);
-      if (kt + 1 < ktiles) fill_step(1, round, kt + 4 < ktiles, r1);
-      if (kt + 2 < ktiles) fill_step(2, round, kt + 5 < ktiles, r2);
-    }
-  } else if (lane == 0) {
-    const int role = warp - GM_FILL_THREADS / 32;
-    if (role < 2 && m0 + role * GM_HM >= M) {
-      // this accumulator's rows lie beyond M (a prompt of at most 128 rows): nothing to multiply; arrive in
-      // step with the other issuing thread so that the stage barriers still count two arrivals per use
-      for (int kt = 0; kt < ktiles; ++kt) {
-        const int s = kt % GM_STAGES, sA = kt % GM_ASTAGES;
-        if (!gm_mbar_wait(&b_full_bar[s], (kt / GM_STAGES) & 1) || !gm_mbar_wait(&full_bar[sA], (kt / GM_ASTAGES) & 1)) fail_s = 1;
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gm_smem_u32(&mma_bar[s])) : "memory");
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(gm_smem_u32(&a_free_bar[sA])) : "memory");
-      }
-    } else if (role < 2) {
-      for (int kt = 0; kt < ktiles; ++kt) issue_mmas(kt, role);
-    } else {
-      // x ring: a stage is refilled as soon as both accumulators' MMAs of four k tiles ago are complete
-      for (int kt = 0; kt < ktiles; ++kt) {
-        if (kt >= GM_ASTAGES && !gm_mbar_wait(&a_free_bar[kt % GM_ASTAGES], ((kt / GM_ASTAGES) - 1) & 1)) {
-          ok = false;
-          fail_s = 1;
-        }
-        issue_a(kt);
-      }
-    }
-  }
-  // ---- drain: the last commit covers every MMA -----------------------------------------------------
-  {
-    const int last = ktiles - 1, s = last % GM_STAGES;
-    if (!gm_mbar_wait(&mma_bar[s], (last / GM_STAGES) & 1)) {
-      ok = false;
-      fail_s = 1;
-    }
-  }
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  __syncthreads();
-  if (fail_s && tid == 0) atomicExch(p.status, 200);
-
-  // ---- epilogue: TMEM -> registers -> fp16 -> shared memory -> global.  A warp reads the TMEM lanes of its
-  // quarter (warp % 4); the four warps of a quarter take 128 of the 512 columns each: columns 0-255 are the
-  // accumulator of tile rows 0-127, columns 256-511 that of rows 128-255.  A thread holds one row, so storing
-  // from registers would scatter 16-byte pieces over 32 rows per instruction; instead the warp parks its
-  // 32 x 128 sub-tile in the (now idle) stage memory and writes it back out row by row, 256 contiguous bytes
-  // per half-warp.
-  // With a K split (few tiles, p.parts > 1) every CTA first stores its fp32 accumulators as partial sums; the
-  // last CTA of a tile to arrive adds the parts in part order (bitwise repeatable) and runs the epilogue.
-  if (warp < GM_FILL_THREADS / 32) {
-    constexpr int ROWB = 128 * 2 + 16;  // bytes per parked row: the pad spreads the lanes' 16-byte stores over the banks
-    const int q = warp & 3, cg = warp >> 2;
-    const int hm = cg >> 1, c_begin = (cg & 1) * 128;
-    unsigned char *park = gm_smem + (size_t)warp * (32 * ROWB);
-    const bool rows_live = !fail_s && m0 + hm * GM_HM + q * 32 < M;  // a warp whose 32 rows all lie beyond M has nothing to store
-    const uint32_t taddr = tmem_acc + ((uint32_t)(q * 32) << 16) + (uint32_t)(hm * GM_BN);
-    const int tile_id = blockIdx.y * gridDim.x + blockIdx.x;
-    // partial sums: [tile][part][16-column chunk][256 rows][16] fp32: a warp's 32 rows of one chunk are 2 KiB of consecutive addresses
-    float *mine = SPLIT ? p.partial + ((size_t)tile_id * p.parts + blockIdx.z) * (GM_BM * GM_BN) + (size_t)(hm * GM_HM + q * 32 + lane) * 16 : nullptr;
-    bool finish = true;
-    if (SPLIT) {
-      if (rows_live) {
-#pragma unroll 2
-        for (int c = 0; c < 128; c += 16) {
-          uint32_t r[16];
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-              : "r"(taddr + c_begin + c));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          float4 *dst = reinterpret_cast<float4 *>(mine + (size_t)((c_begin + c) / 16) * (GM_BM * 16));
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            __stcg(dst + j, make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]), __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3])));
-        }
-      }
-      __threadfence();
-      asm volatile("bar.sync 1, %0;" ::"n"(GM_FILL_THREADS) : "memory");
-      if (tid == 0) {
-        const unsigned old = atomicAdd(p.counters + tile_id, 1u);
-        const int last = old == (unsigned)(p.parts - 1);
-        if (last) p.counters[tile_id] = 0;  // ready for the next launch
-        last_s = last;
-      }
-      asm volatile("bar.sync 1, %0;" ::"n"(GM_FILL_THREADS) : "memory");
-      finish = last_s != 0;
-      if (finish) __threadfence();
-    }
-    if (finish && rows_live) {
-      const float *all = SPLIT ? p.partial + (size_t)tile_id * p.parts * (GM_BM * GM_BN) + (size_t)(hm * GM_HM + q * 32 + lane) * 16 : nullptr;
-#pragma unroll 2
-      for (int c = 0; c < 128; c += 16) {
-        float v[16];
-        if (SPLIT) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = 0.f;
-          for (int pt0 = 0; pt0 < p.parts; pt0 += 4) {  // four parts' loads in flight together, added in part order
-            float4 a[4][4];
-#pragma unroll
-            for (int pp = 0; pp < 4; ++pp) {
-              const float4 *src = reinterpret_cast<const float4 *>(all + (size_t)(pt0 + pp) * (GM_BM * GM_BN) + (size_t)((c_begin + c) / 16) * (GM_BM * 16));
-#pragma unroll
-              for (int j = 0; j < 4; ++j) a[pp][j] = pt0 + pp < p.parts ? __ldcg(src + j) : make_float4(0.f, 0.f, 0.f, 0.f);
-            }
-#pragma unroll
-            for (int pp = 0; pp < 4; ++pp)
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                v[4 * j] += a[pp][j].x;
-                v[4 * j + 1] += a[pp][j].y;
-                v[4 * j + 2] += a[pp][j].z;
-                v[4 * j + 3] += a[pp][j].w;
-              }
-          }
-        } else {
-          uint32_t r[16];
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-                "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-              : "r"(taddr + c_begin + c));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-        }
-        uint4 h0, h1;
-        h0.x = h22u(__floats2half2_rn(v[0], v[1]));
-        h0.y = h22u(__floats2half2_rn(v[2], v[3]));
-        h0.z = h22u(__floats2half2_rn(v[4], v[5]));
-        h0.w = h22u(__floats2half2_rn(v[6], v[7]));
-        h1.x = h22u(__floats2half2_rn(v[8], v[9]));
-        h1.y = h22u(__floats2half2_rn(v[10], v[11]));
-        h1.z = h22u(__floats2half2_rn(v[12], v[13]));
-        h1.w = h22u(__floats2half2_rn(v[14], v[15]));
-        *reinterpret_cast<uint4 *>(park + lane * ROWB + c * 2) = h0;
-        *reinterpret_cast<uint4 *>(park + lane * ROWB + c * 2 + 16) = h1;
+        const uint4 wa = *reinterpret_cast<const uint4 *>(words + ps * GS_P_BYTES), wb = *reinterpret_cast<const uint4 *>(words + ps * GS_P_BYTES + 16);
+        w[0] = wa.x, w[1] = wa.y, w[2] = wa.z, w[3] = wa.w, w[4] = wb.x, w[5] = wb.y, w[6] = wb.z, w[7] = wb.w;
+        sv = *reinterpret_cast<const uint4 *>(scale + ps * GS_P_BYTES);
       }
       __syncwarp();
-      const int piece = lane & 15;                       // 16-byte piece (8 columns) of a parked row
-      const int col = n0 + c_begin + piece * 8;
-      if (col < N) {                                     // N is a multiple of 8: a piece is inside or outside as a whole
-#pragma unroll 4
-        for (int rr = 0; rr < 32; rr += 2) {
-          const int rl = rr + (lane >> 4);
-          const int row = m0 + hm * GM_HM + q * 32 + rl;
-          const uint4 v = *reinterpret_cast<const uint4 *>(park + rl * ROWB + piece * 16);
-          if (row < M) *reinterpret_cast<uint4 *>(p.out + (size_t)row * N + col) = v;
+      if (lane == 0) gs_arrive(b_pempty + 8 * ps);
+      if constexpr (TMEM) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t o[16];  // four words: 32 values in k order, two per column of tensor memory
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            uint32_t k04, k15, k26, k37;
+            dequant(w[4 * half + r], u2h2(sv.x), k04, k15, k26, k37);
+            o[4 * r] = __byte_perm(k04, k15, 0x5410);
+            o[4 * r + 1] = __byte_perm(k26, k37, 0x5410);
+            o[4 * r + 2] = __byte_perm(k04, k15, 0x7632);
+            o[4 * r + 3] = __byte_perm(k26, k37, 0x7632);
+          }
+          gs_st16(tmem_w + a * 32 + ((uint32_t)(q * 32) << 16) + ws * GS_W_COLS + half * 16, o);
+        }
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      } else {
+        uint32_t o[8][4];  // [k][column pair]
+        const uint32_t sc[4] = {sv.x, sv.y, sv.z, sv.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {  // k 0..3 are the low halves of the words, k 4..7 the high ones
+          dequant(__byte_perm(w[2 * j], w[2 * j + 1], 0x5410), u2h2(sc[j]), o[0][j], o[1][j], o[2][j], o[3][j]);
+          dequant(__byte_perm(w[2 * j], w[2 * j + 1], 0x7632), u2h2(sc[j]), o[4][j], o[5][j], o[6][j], o[7][j]);
+        }
+        unsigned char *dst = smem + ws * GS_W_BYTES + (lane >> 3) * (GS_BK * 128) + r8 * 1024;  // block of 64 columns, atom of 8 k
+#pragma unroll
+        for (int k = 0; k < 8; ++k) *reinterpret_cast<uint4 *>(dst + k * 128 + (((lane & 7) ^ k) << 4)) = make_uint4(o[k][0], o[k][1], o[k][2], o[k][3]);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic-proxy writes -> visible to the tensor core
+      }
+      __syncwarp();
+      if (lane == 0) gs_arrive(bar_of(b_full, u));
+      ws += 2;
+      if (ws >= dw) ws -= dw;
+      ps += 2;
+      if (ps >= dp) ps -= dp, pph ^= 1;
+    }
+    if (!good) fail_s = 1;
+  }
+  pdl_wait();  // (long satisfied) out may still have been in use
+  // ---- all MMAs of this CTA are done, its shared memory is idle -----------------------------------------------------
+  if (!gs_wait(b_done, 0)) fail_s = 1;
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  __syncthreads();
+  const bool failed = fail_s != 0;
+
+  // Epilogue.  A warp reads the tensor-memory lanes of its quarter (warp % 4): lane = column of an accumulator's run; the
+  // four warps of a quarter share the mt accumulator columns (= rows of x) in chunks of 16.
+  const int q = warp & 3, sub = warp >> 2;
+  const int chunks = mt / 16;
+  const uint32_t lanes = (uint32_t)(q * 32) << 16;
+  if (parts == 1) {
+    // A thread holds a column: results are parked row by row in the idle operand memory and leave as whole 512-byte rows
+    // (SILU: 256).  (Two bytes per lane straight to global memory were 5-10% of a large call.)
+    constexpr int ROW_VECS = (SILU ? GS_BN / 2 : GS_BN) / 8;
+    if (warp < GS_DQ_WARPS && !failed) {
+      for (int i = sub; i < chunks; i += 4) {
+        if (m0 + i * 16 >= p.M) break;
+        float v[16], w[16];
+        gs_ld16(tmem + i * 16 + lanes, v);
+        gs_ld16(tmem + acc1 + i * 16 + lanes, w);
+        __half *o = reinterpret_cast<__half *>(smem + (size_t)i * 16 * GS_ROWB) + q * 32 + lane;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          if (SILU) {
+            o[j * (GS_ROWB / 2)] = __float2half_rn(gs_silu_mul(v[j], w[j]));
+          } else {
+            o[j * (GS_ROWB / 2)] = __float2half_rn(v[j]);
+            o[j * (GS_ROWB / 2) + 128] = __float2half_rn(w[j]);
+          }
+        }
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(GS_DQ_THREADS) : "memory");
+      const int piece = tid % ROW_VECS, n = n0 + piece * 8, rows = min(mt, p.M - m0);
+      if (n < p.n_out)  // n_out is a multiple of 8: a piece is inside or outside as a whole
+        for (int m = tid / ROW_VECS; m < rows; m += GS_DQ_THREADS / ROW_VECS)
+          *reinterpret_cast<uint4 *>(p.out + (size_t)(m0 + m) * p.n_out + n) = *reinterpret_cast<const uint4 *>(smem + (size_t)m * GS_ROWB + piece * 16);
+    }
+  } else {
+    // The chunks are owned by the ranks in consecutive runs.  Inbox of a CTA: [own chunk][source rank][accumulator][row
+    // quad][column][4] fp32, 16 KiB per chunk and rank.  When they do not fit together, half of them go first.
+    const int rounds = ((chunks + parts - 1) / parts) * parts * GS_ITEM_BYTES <= GS_SMEM_LIMIT - 1024 ? 1 : 2;
+    for (int round = 0; round < rounds; ++round) {
+      const int c0 = chunks * round / rounds, count = chunks * (round + 1) / rounds - c0;
+      auto first = [&](int r) { return count * r / parts; };
+      const int own0 = first(part), own = first(part + 1) - own0;
+      cluster.sync();  // every CTA's shared memory is idle
+      if (warp < GS_DQ_WARPS) {
+        int owner = 0;
+        for (int i = sub >> 1; i < count; i += 2) {  // two warps of a quarter per accumulator
+          while (first(owner + 1) <= i) ++owner;
+          const int a = sub & 1;
+          float v[16];
+          gs_ld16(tmem + a * acc1 + (c0 + i) * 16 + lanes, v);
+          float4 *dst = reinterpret_cast<float4 *>(cluster.map_shared_rank(smem, owner) + ((i - first(owner)) * parts + part) * GS_ITEM_BYTES) + a * 512 + q * 32 + lane;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dst[j * 128] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        }
+      }
+      cluster.sync();
+      if (warp < GS_DQ_WARPS && !failed) {
+        for (int i = 0; i < own; ++i) {  // thread = row quad tid / 128 of a chunk, column tid % 128 of both accumulators
+          const int m = m0 + (c0 + own0 + i) * 16 + (tid >> 7) * 4, n = n0 + (tid & 127);
+          const float4 *src = reinterpret_cast<const float4 *>(smem + (size_t)i * parts * GS_ITEM_BYTES) + tid;
+          float4 t = src[0], u = src[512];
+          for (int r = 1; r < parts; ++r) {
+            const float4 a = src[r * (GS_ITEM_BYTES / 16)], b = src[r * (GS_ITEM_BYTES / 16) + 512];
+            t.x += a.x, t.y += a.y, t.z += a.z, t.w += a.w;
+            u.x += b.x, u.y += b.y, u.z += b.z, u.w += b.w;
+          }
+          const float f[4] = {t.x, t.y, t.z, t.w}, g[4] = {u.x, u.y, u.z, u.w};
+          __half *o = p.out + (size_t)m * p.n_out + n;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (m + j < p.M) {
+              if (SILU) {
+                if (n < p.n_out) o[(size_t)j * p.n_out] = __float2half_rn(gs_silu_mul(f[j], g[j]));
+              } else {
+                if (n < p.n_out) o[(size_t)j * p.n_out] = __float2half_rn(f[j]);
+                if (n + 128 < p.n_out) o[(size_t)j * p.n_out + 128] = __float2half_rn(g[j]);
+              }
+            }
         }
       }
     }
   }
-  (void)ok;
+  if (failed && tid == 0) atomicExch(p.status, 210);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(2 * GM_BN) : "memory");
+  if (warp == GS_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(512) : "memory");
 }
 
-// Library-owned scratch for K-split launches: [counters, zero between launches][partial sums]; at most one
-// 256 x 256 fp32 tile per SM (37 MiB on 148 SMs).
-constexpr size_t GEMM_COUNTER_BYTES = 1024;
-static int gemm_scratch(size_t bytes, void **out) { return library_buffer(LIB_BUF_GEMM, bytes, 0, GEMM_COUNTER_BYTES, out); }
+// Clusters of `parts` CTAs of this kernel that are resident at once on the current device (asked once per device).
+static int gs_clusters(int parts) {
+  static std::atomic<int> known[64][GS_MAX_PARTS + 1];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = known[dev][parts].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(parts, 1, 1);
+    cfg.blockDim = dim3(GS_THREADS, 1, 1);
+    cfg.dynamicSmemBytes = GS_SMEM_LIMIT;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = parts;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, w4a16_gemm_tcgen05_kernel<false, true>, &cfg) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      n = -1;
+    }
+    known[dev][parts].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+
+static int gemm_launch(const void *x, const int32_t *qweight, const void *scales, void *out, int M, int K, int N, int group, bool silu, cudaStream_t stream) {
+  AB200_REQUIRE(x && qweight && scales && out, "w4a16_gemm: null pointer");
+  AB200_REQUIRE(M > 0 && N > 0 && N % 8 == 0, "w4a16_gemm: M=%d must be positive, N=%d a positive multiple of 8", M, N);
+  AB200_REQUIRE(K > 0 && K % GS_BK == 0, "w4a16_gemm: K=%d must be a positive multiple of %d", K, GS_BK);
+  AB200_REQUIRE(group >= GS_BK && group % GS_BK == 0 && K % group == 0, "w4a16_gemm: group=%d must be a multiple of %d dividing K", group, GS_BK);
+  AB200_REQUIRE(aligned16(x) && aligned16(qweight) && aligned16(scales) && aligned16(out), "w4a16_gemm: pointers must be 16-byte aligned");
+  int *status = kernel_error_ptr();
+  AB200_REQUIRE(status != nullptr, "w4a16_gemm: cannot resolve the status word");
+  typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
+                               const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  EncodeFn enc = reinterpret_cast<EncodeFn>(tensor_map_encoder());
+  if (!enc) return fail(AB200_EUNSUPPORTED, "w4a16_gemm: this driver has no cuTensorMapEncodeTiled");
+  AB200_CUDA(cudaFuncSetAttribute(w4a16_gemm_tcgen05_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM_LIMIT));  // gs_clusters asks about it
+
+  // Row tiles: at least M / 256; more and narrower ones when that fills the last round of CTAs better.  K split, when the
+  // tiles leave SMs idle: as many parts as keep every tile's cluster resident at once (a cluster lies within one GPC, so
+  // this is not SMs / parts), each of at least 4 units.  A unit costs about what was measured for the two
+  // forms; a tile costs its start and epilogue, a split the exchange of its rows.
+  const int tiles_n = silu ? (N / 2 + GS_BN / 2 - 1) / (GS_BN / 2) : (N + GS_BN - 1) / GS_BN, units = K / GS_BK, sms = sm_count();
+  auto rows_of = [&](int tiles_m) { return ((M + tiles_m - 1) / tiles_m + 15) / 16 * 16; };
+  auto parts_of = [&](long tiles) {
+    int parts = GS_MAX_PARTS;
+    while (parts > 1 && (parts > units / 4 || tiles * parts > sms || tiles > gs_clusters(parts))) --parts;
+    return parts;
+  };
+  auto cost = [&](int tiles_m) {
+    const long tiles = (long)tiles_n * tiles_m, rounds = (tiles + sms - 1) / sms;
+    const int rows = rows_of(tiles_m), unit = rows <= GS_TMEM_MT ? 650 + 2 * rows : 700 + 3 * rows, parts = parts_of(tiles);
+    return rounds * ((long)((units + parts - 1) / parts) * unit + GS_TILE_CYCLES + (parts > 1 ? GS_SPLIT_CYCLES + rows * GS_SPLIT_ROW_CYCLES : 0));
+  };
+  const int least = (M + GS_MAX_MT - 1) / GS_MAX_MT;
+  int tiles_m = least;
+  long best = cost(least);
+  for (int t = least + 1; t <= least + 8 && t <= (M + 15) / 16; ++t)
+    if (const long c = cost(t); c < best) best = c, tiles_m = t;
+  const int mt = rows_of(tiles_m), parts = parts_of((long)tiles_n * tiles_m);
+
+  auto encode = [&](CUtensorMap *tm, CUtensorMapDataType type, const void *base, int elt, cuuint64_t inner, cuuint64_t outer, int box_inner, int box_outer,
+                    CUtensorMapSwizzle swizzle) {
+    const cuuint64_t dims[2] = {inner, outer}, strides[1] = {inner * elt};
+    const cuuint32_t box[2] = {(cuuint32_t)box_inner, (cuuint32_t)box_outer}, estr[2] = {1, 1};
+    return enc(tm, type, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUtensorMap tm_x, tm_w, tm_s;
+  CUresult r = encode(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, 2, K, M, GS_BK, mt, CU_TENSOR_MAP_SWIZZLE_128B);
+  if (r == CUDA_SUCCESS) r = encode(&tm_w, CU_TENSOR_MAP_DATA_TYPE_INT32, qweight, 4, N, K / 8, 128, GS_BK / 8, CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (r == CUDA_SUCCESS) r = encode(&tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, scales, 2, N, K / group, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE);
+  if (r != CUDA_SUCCESS) return fail(AB200_ECUDA, "w4a16_gemm: cuTensorMapEncodeTiled failed with %d", (int)r);
+
+  GemmParams p{(__half *)out, M, K, N, group, mt, silu ? N / 2 : 128, silu ? N / 2 : N, 0, 0, 0, status};
+  const bool in_tmem = mt <= GS_TMEM_MT;
+  const int xb = mt * GS_BK * 2, w_cols = 512 - 2 * ((mt + 31) & ~31);
+  p.dw = !in_tmem ? 3 : w_cols / GS_W_COLS < GS_MAX_DW ? w_cols / GS_W_COLS : GS_MAX_DW;
+  p.dx = in_tmem ? GS_MAX_DX : 3;
+  const int room = GS_SMEM_LIMIT - 1024 - p.dx * xb - (in_tmem ? 0 : p.dw * GS_W_BYTES);  // for at least 3 packed units (mt = 256), 9 in tensor memory's form
+  p.dp = room / GS_P_BYTES < GS_MAX_DP ? room / GS_P_BYTES : GS_MAX_DP;
+  auto kern = silu ? (in_tmem ? w4a16_gemm_tcgen05_kernel<true, true> : w4a16_gemm_tcgen05_kernel<true, false>) : (in_tmem ? w4a16_gemm_tcgen05_kernel<false, true> : w4a16_gemm_tcgen05_kernel<false, false>);
+  AB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, GS_SMEM_LIMIT));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles_n * parts, tiles_m, 1);
+  cfg.blockDim = dim3(GS_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = GS_SMEM_LIMIT;  // one CTA per SM; the inboxes of a K split use all of it
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = parts;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  AB200_CUDA(cudaLaunchKernelEx(&cfg, kern, tm_x, tm_w, tm_s, p));
+  return AB200_OK;
+}
 
 }  // namespace ab200
 
@@ -450,46 +537,11 @@ extern "C" int ab200_w4a16_gemm(const void *x, const int32_t *qweight, const voi
   clear_error();
   AB200_REQUIRE(x && qweight && scales && out, "w4a16_gemm: null pointer");
   if (dtype != AB200_F16) return fail(AB200_EUNSUPPORTED, "w4a16_gemm: the tensor-core path is built for float16 (dtype %d given)", dtype);
-  AB200_REQUIRE(M > 0 && N > 0 && N % 8 == 0, "w4a16_gemm: M=%d must be positive, N=%d a positive multiple of 8", M, N);
-  AB200_REQUIRE(K > 0 && K % GM_BK == 0, "w4a16_gemm: K=%d must be a positive multiple of %d", K, GM_BK);
-  AB200_REQUIRE(group >= GM_BK && group % GM_BK == 0 && K % group == 0, "w4a16_gemm: group=%d must be a multiple of %d dividing K", group, GM_BK);
-  AB200_REQUIRE(aligned16(x) && aligned16(qweight) && aligned16(scales) && aligned16(out), "w4a16_gemm: pointers must be 16-byte aligned");
-  int *status = kernel_error_ptr();
-  AB200_REQUIRE(status != nullptr, "w4a16_gemm: cannot resolve the status word");
-  // Few tiles (a short prompt): split K over the idle SMs, at most 4 ranges (the last CTA of a tile adds all
-  // parts, one batch of loads per 16 columns) of at least 8 k tiles each
-  const int tiles = ((N + GM_BN - 1) / GM_BN) * ((M + GM_BM - 1) / GM_BM), G = sm_count();
-  int parts = G / tiles;
-  if (parts > 4) parts = 4;
-  if (parts > (K / GM_BK) / 8) parts = (K / GM_BK) / 8;
-  if (parts < 1) parts = 1;
-  void *scratch = nullptr;
-  if (parts > 1) {
-    if (int rc = gemm_scratch(GEMM_COUNTER_BYTES + (size_t)tiles * parts * GM_BM * GM_BN * sizeof(float), &scratch)) return rc;
-  }
-  GemmParams p{(const __half *)x, qweight, (const __half *)scales, (__half *)out, M, K, N, group, status, parts,
-               scratch ? reinterpret_cast<float *>(reinterpret_cast<unsigned char *>(scratch) + GEMM_COUNTER_BYTES) : nullptr,
-               reinterpret_cast<unsigned *>(scratch)};
-  typedef CUresult (*EncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *,
-                               const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                               CUtensorMapFloatOOBfill);
-  EncodeFn enc = reinterpret_cast<EncodeFn>(tensor_map_encoder());
-  if (!enc) return fail(AB200_EUNSUPPORTED, "w4a16_gemm: this driver has no cuTensorMapEncodeTiled");
-  CUtensorMap tm_x;
-  {
-    const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)M};
-    const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
-    const cuuint32_t box[2] = {GM_BK, GM_HM}, estr[2] = {1, 1};
-    const CUresult r = enc(&tm_x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(AB200_ECUDA, "w4a16_gemm: cuTensorMapEncodeTiled(x) failed with %d", (int)r);
-  }
-  const size_t smem = (size_t)GM_ASTAGES * GM_A_BYTES + (size_t)GM_STAGES * GM_B_BYTES + 1024;
-  AB200_CUDA(cudaFuncSetAttribute(w4a16_gemm_tcgen05_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  AB200_CUDA(cudaFuncSetAttribute(w4a16_gemm_tcgen05_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const dim3 grid((N + GM_BN - 1) / GM_BN, (M + GM_BM - 1) / GM_BM, parts);
-  if (parts > 1) w4a16_gemm_tcgen05_kernel<true><<<grid, GM_THREADS, smem, (cudaStream_t)stream>>>(tm_x, p);
-  else w4a16_gemm_tcgen05_kernel<false><<<grid, GM_THREADS, smem, (cudaStream_t)stream>>>(tm_x, p);
-  AB200_CHECK_LAUNCH("w4a16_gemm");
-  return AB200_OK;
+  return gemm_launch(x, qweight, scales, out, M, K, N, group, false, (cudaStream_t)stream);
+}
+
+extern "C" int ab200_w4a16_gemm_silu(const void *x, const int32_t *qweight, const void *scales, void *out, int M, int K, int N, int group, void *stream) {
+  clear_error();
+  AB200_REQUIRE(N % 16 == 0, "w4a16_gemm_silu: N=%d must be twice a multiple of 8", N);
+  return gemm_launch(x, qweight, scales, out, M, K, N, group, true, (cudaStream_t)stream);
 }

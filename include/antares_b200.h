@@ -165,13 +165,13 @@ int ab200_residual_add(float *x_f32, const float *partial_f32, int n, void *stre
 
 /* Prefill contraction on tensor cores (tcgen05 + TMEM): same arithmetic, any M >= 1 (fp16, K a
  * multiple of 64, group a multiple of 64 dividing K, N a multiple of 8).  Replaces the same
- * exported op called with a leading M axis.  When the problem has fewer 256 x 256 output tiles
- * than half the SMs, K is split over the idle SMs and the partial sums pass through a
- * library-owned per-device scratch (at most 37 MiB), allocated by the first such call on a
- * device: make that call outside stream capture, and do not let two such calls overlap on
- * different streams. */
+ * exported op called with a leading M axis.  Uses no scratch. */
 int ab200_w4a16_gemm(const void *x, const int32_t *qweight, const void *scales, void *out, int M,
                      int K, int N, int group, int dtype, void *stream);
+/* The same with weights [gate | up] (N = 2F, N a multiple of 16): out [M, F] = silu(gate) * up of the
+ * fp16-rounded projections, i.e. ab200_w4a16_gemm followed by ab200_silu_mul_rows in one pass. */
+int ab200_w4a16_gemm_silu(const void *x, const int32_t *qweight, const void *scales, void *out, int M,
+                          int K, int N, int group, void *stream);
 
 /* ---- elementwise / reduction operators ---------------------------------------------------- */
 
