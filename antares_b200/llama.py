@@ -344,7 +344,7 @@ class LlamaInt4Decoder:
         d, dl, f, dev = self.cfg.dim, self.dl, self.fl, self.dev
         h16 = lambda *shape: torch.empty(*shape, dtype=torch.float16, device=dev)
         return dict(x=torch.empty(T, d, dtype=torch.float32, device=dev), xb=h16(T, d), vqk=h16(T, 3 * dl), q=h16(T, dl), att=h16(T, dl),
-                    o=h16(T, d), gu=h16(T, 2 * f), hh=h16(T, f))
+                    o=h16(T, d), hh=h16(T, f))
 
     def _prefill_pass(self, T, b):
         """The launches of one batched prompt pass on torch's current stream; reads self.prompt[:T], pos = 0."""
@@ -352,15 +352,25 @@ class LlamaInt4Decoder:
         st = torch.cuda.current_stream().cuda_stream
         toks = self.prompt[:T]
         d, f = cfg.dim, self.fl
-        x, xb, vqk, q, att, o, gu, hh = b["x"], b["xb"], b["vqk"], b["q"], b["att"], b["o"], b["gu"], b["hh"]
+        x, xb, vqk, q, att, o, hh = b["x"], b["xb"], b["vqk"], b["q"], b["att"], b["o"], b["hh"]
         call("ab200_embed_rows", self.embed.data_ptr(), toks.data_ptr(), x.data_ptr(), T, d, cfg.vocab, st)
 
         def gemm(a, l, k, out):
             qw, sc = self._ref_layout(l, k)
             call("ab200_w4a16_gemm", a.data_ptr(), qw.data_ptr(), sc.data_ptr(), out.data_ptr(), T, qw.shape[0] * 8, qw.shape[1], cfg.group, 0, st)
 
+        def residual(norm_w):
+            """x += o, and the rows the next projection reads: their RMSNorm, in the same pass."""
+            if self.world > 1:
+                self.comm.all_reduce_sum_(o)
+            if norm_w is None:
+                call("ab200_residual_add_f16", x.data_ptr(), o.data_ptr(), T * d, st)
+            else:
+                call("ab200_residual_rmsnorm", x.data_ptr(), o.data_ptr(), norm_w.data_ptr(), xb.data_ptr(), T, d, cfg.eps, st)
+
+        if self.layers:
+            call("ab200_rmsnorm", x.data_ptr(), 1, self.layers[0]["att_norm"].data_ptr(), xb.data_ptr(), T, d, cfg.eps, st)
         for l, w in enumerate(self.layers):
-            call("ab200_rmsnorm", x.data_ptr(), 1, w["att_norm"].data_ptr(), xb.data_ptr(), T, d, cfg.eps, st)
             gemm(xb, l, "vqk", vqk)
             if self.page_table is None:
                 call("ab200_rope_kv_store_rows", vqk.data_ptr(), self.inv_freq.data_ptr(), self.pos.data_ptr(), q.data_ptr(),
@@ -374,16 +384,11 @@ class LlamaInt4Decoder:
                 call("ab200_attention_prefill_paged", q.data_ptr(), self.k_cache[l].data_ptr(), self.v_cache[l].data_ptr(), att.data_ptr(),
                      self.pos.data_ptr(), T, cfg.max_seq, self.hl, cfg.head_dim, self.dl, self.att_scale, pt, pr, st)
             gemm(att, l, "o", o)
-            if self.world > 1:
-                self.comm.all_reduce_sum_(o)
-            call("ab200_residual_add_f16", x.data_ptr(), o.data_ptr(), T * d, st)
-            call("ab200_rmsnorm", x.data_ptr(), 1, w["ffn_norm"].data_ptr(), xb.data_ptr(), T, d, cfg.eps, st)
-            gemm(xb, l, "gu", gu)
-            call("ab200_silu_mul_rows", gu.data_ptr(), hh.data_ptr(), T, f, st)
+            residual(w["ffn_norm"])
+            qw, sc = self._ref_layout(l, "gu")   # gate | up, silu(gate) * up on the way out
+            call("ab200_w4a16_gemm_silu", xb.data_ptr(), qw.data_ptr(), sc.data_ptr(), hh.data_ptr(), T, d, 2 * f, cfg.group, st)
             gemm(hh, l, "down", o)
-            if self.world > 1:
-                self.comm.all_reduce_sum_(o)
-            call("ab200_residual_add_f16", x.data_ptr(), o.data_ptr(), T * d, st)
+            residual(self.layers[l + 1]["att_norm"] if l + 1 < len(self.layers) else None)
         # classifier on the last token only, then the same bookkeeping as a decode step at pos = T - 1
         self.x.copy_(x[T - 1])
         self.pos.fill_(T - 1)

@@ -322,6 +322,10 @@ int ab200_attention_prefill(const void *q_f16, const void *k_cache_f16, const vo
 int ab200_silu_mul_rows(const void *gate_up_f16, void *out_f16, int rows, int n, void *stream);
 /* x_f32[i] += y_f16[i] (residual update after a prefill GEMM). */
 int ab200_residual_add_f16(float *x_f32, const void *y_f16, size_t n, void *stream);
+/* The same for [rows, cols], and out_f16 = RMSNorm of the updated rows (weight fp16 [cols]) in the same
+ * pass; cols % 8 == 0, cols <= 16384. */
+int ab200_residual_rmsnorm(float *x_f32, const void *y_f16, const void *weight_f16, void *out_f16,
+                           int rows, int cols, float eps, void *stream);
 
 /* One-shot hint for the calling thread's NEXT fp16 ab200_w4a16_gemv* call: while that kernel
  * streams its own weights, one thread per CTA also asks for the two byte ranges (normally the

@@ -147,3 +147,20 @@ def test_attention_against_the_reference_samples_open_statement(cuda, S):
                                  torch.tensor([S], dtype=torch.int32, device=cuda), att_f)
         err = np.abs(y.float().cpu().numpy() - ref).max() / np.abs(ref).max()
         assert err <= tol, (dt, err)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 2048), (5, 4096), (700, 4104), (2, 16384)])
+def test_residual_update_with_the_next_norm(rows, cols):
+    """One pass = the residual add followed by RMSNorm, bit for bit."""
+    import torch
+    from antares_b200._lib import call
+    g = torch.Generator(device="cuda").manual_seed(rows * cols)
+    x = torch.randn(rows, cols, generator=g, device="cuda")
+    y, w = torch.randn(rows, cols, generator=g, device="cuda").half(), torch.randn(cols, generator=g, device="cuda").half()
+    st = torch.cuda.current_stream().cuda_stream
+    apart, want, out = x.clone(), torch.empty_like(y), torch.empty_like(y)
+    call("ab200_residual_add_f16", apart.data_ptr(), y.data_ptr(), rows * cols, st)
+    call("ab200_rmsnorm", apart.data_ptr(), 1, w.data_ptr(), want.data_ptr(), rows, cols, 1e-6, st)
+    call("ab200_residual_rmsnorm", x.data_ptr(), y.data_ptr(), w.data_ptr(), out.data_ptr(), rows, cols, 1e-6, st)
+    assert torch.equal(x, apart) and torch.equal(out, want)
