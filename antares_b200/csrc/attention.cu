@@ -456,7 +456,10 @@ extern "C" int ab200_attention_fused_paged(const void *vqk_f16, const float *inv
   return attention_fused_impl(vqk_f16, inv_freq, pos_dev, k_cache_f16, v_cache_f16, out_f16, H, D, kv_stride, max_seq, scale, page_table, page_rows, stream);
 }
 
-constexpr int ATT_PREFILL_TC_ROWS = 9;
+// From how many rows on a prompt goes through the tensor-core kernel.  us, 32 heads, from position 0, the single-query
+// kernel per row against that one: 16 rows 4.2 / 10.9, 32 rows 7.7 / 11.0, 64 rows 14.6 / 10.5, 128 rows 33 / 12.  (The
+// position is a device value, so the rule cannot look at it: behind 500 cached rows the lines cross below 1 row.)
+constexpr int ATT_PREFILL_TC_ROWS = 41;
 
 // Causal attention of `rows` consecutive tokens over a cache that already holds their keys and
 // values: query row r (position *pos0_dev + r) attends cache rows 0 .. *pos0_dev + r.  The batched

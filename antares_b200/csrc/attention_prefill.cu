@@ -19,6 +19,10 @@
 // resident per SM and one's MMAs run under the other's softmax.  Query tiles are issued last row first: the
 // longest CTAs start first.
 //
+// What bounds it: the softmax warps.  A tile of a CTA takes 2200 cycles, 1250 of them exponentials, row sums and the split
+// of P (two softmax warps share a scheduler's 4 exponentials a cycle: 1024 cycles); its 16 MMAs wait for that.
+// 32 heads, 2000 rows: 78 us (4162 with the single-query kernel once per row); 128 rows: 12 us (33).
+//
 // Values of V that are not finite: a masked or underflowed probability is exactly 0 in the MMA, and 0 * inf
 // would reach rows that never attend to that key.  The loading warps look at every V tile; a CTA that saw one
 // recomputes its rows with fp32 code that touches only the keys a row attends to (attend_row below).

@@ -183,8 +183,7 @@ __device__ __forceinline__ void vm_store(void *p, bool f16, size_t i, unsigned s
 }
 
 // Runs n instructions for EN elements; scalar(kind, index) and vector(kind, index, b) fetch operands, `first` is the
-// first input.  code: in shared memory (from the kernel's parameters every word was a miss in the small constant cache).
-// stack: this thread's column of [slot][VM_E / 4][threads] float4.
+// first input.  stack: this thread's column of [slot][VM_E / 4][threads] float4.
 // Decoding is a chain of dependent loads and branches, which is what a short program spends its time on: the next word is
 // read ahead, and the commonest operations are tested before the jump table, with a scalar or the first input without a
 // copy of the operand.

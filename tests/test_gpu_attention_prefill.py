@@ -51,7 +51,7 @@ def _close(got, want, v, score=0.0):
 
 
 # edges of the query tile (128) and the key tile (64), both sides of the row rule, one row, prompts behind a filled cache
-@pytest.mark.parametrize("rows,pos0,max_seq", [(1, 0, 64), (8, 3, 64), (9, 0, 16), (16, 0, 16), (17, 46, 63), (63, 0, 64), (64, 1, 65), (65, 0, 80), (127, 0, 200),
+@pytest.mark.parametrize("rows,pos0,max_seq", [(1, 0, 64), (8, 3, 64), (16, 0, 16), (40, 0, 64), (41, 0, 64), (41, 22, 63), (41, 900, 941), (63, 0, 64), (64, 1, 65), (65, 0, 80), (127, 0, 200),
                                                (128, 0, 128), (129, 0, 129), (200, 300, 512), (451, 0, 451), (30, 1000, 1030)])
 @pytest.mark.parametrize("sharp", [1.0, 24.0])  # 24: scores spread over hundreds, the running maximum moves often
 def test_prefill_attention(rows, pos0, max_seq, sharp):
