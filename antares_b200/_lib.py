@@ -55,6 +55,7 @@ SIGNATURES = {
     "ab200_w4a16_gemv_tiled_allreduce": [_vp, _i, _vp, _vp, _vp, _i, _i, _i, _vp, _i, _i, _i, _vp],
     "ab200_w4a16_gemv_tiled_allreduce_emulated": [_vp, _i, _vp, _vp, _vp, _vp, _i, _vp, _i, _i, _vp, _vp],
     "ab200_w4a16_gemm": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
+    "ab200_w4a16_gemm_early": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _vp],
     "ab200_w4a16_gemm_silu": [_vp, _vp, _vp, _vp, _i, _i, _i, _i, _vp],
     "ab200_sigmoid": [_vp, _vp, _sz, _i, _vp],
     "ab200_rmsnorm_vsum": [_vp, _vp, _vp, _vp, _sz, _f, _f, _i, _vp],

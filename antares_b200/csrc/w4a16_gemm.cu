@@ -69,6 +69,7 @@ struct GemmParams {
   int n_out;   // columns of out
   int dx, dw, dp;  // ring depths
   int *status;
+  int early;   // launched while the kernel before runs: weights and scales date from before it
 };
 
 __device__ __forceinline__ uint32_t gs_smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -176,7 +177,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(gs_smem_u32(&tmem_s)), "n"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  pdl_launch_dependents();
+  if (p.early) pdl_launch_dependents();
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -204,7 +205,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
     __syncwarp();
   } else if (warp == GS_X_WARP) {
     if (gs_elect()) {  // x tiles
-      pdl_wait();      // x comes from the kernel before this one; weights and scales are constant and already on their way
+      pdl_wait();      // x comes from the kernel before this one; weights and scales may be on their way already (p.early)
       for (int u = 0, slot = 0; u < n_units; ++u) {
         if (u >= dx && !gs_wait(bar_of(b_used, u - dx), phase_of(u - dx))) {
           good = false;
@@ -451,7 +452,7 @@ static int gs_clusters(int parts) {
   return n;
 }
 
-static int gemm_launch(const void *x, const int32_t *qweight, const void *scales, void *out, int M, int K, int N, int group, bool silu, cudaStream_t stream) {
+static int gemm_launch(const void *x, const int32_t *qweight, const void *scales, void *out, int M, int K, int N, int group, bool silu, bool early, cudaStream_t stream) {
   AB200_REQUIRE(x && qweight && scales && out, "w4a16_gemm: null pointer");
   AB200_REQUIRE(M > 0 && N > 0 && N % 8 == 0, "w4a16_gemm: M=%d must be positive, N=%d a positive multiple of 8", M, N);
   AB200_REQUIRE(K > 0 && K % GS_BK == 0, "w4a16_gemm: K=%d must be a positive multiple of %d", K, GS_BK);
@@ -501,7 +502,7 @@ static int gemm_launch(const void *x, const int32_t *qweight, const void *scales
   if (r == CUDA_SUCCESS) r = encode(&tm_s, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, scales, 2, N, K / group, 128, 1, CU_TENSOR_MAP_SWIZZLE_NONE);
   if (r != CUDA_SUCCESS) return fail(AB200_ECUDA, "w4a16_gemm: cuTensorMapEncodeTiled failed with %d", (int)r);
 
-  GemmParams p{(__half *)out, M, K, N, group, mt, silu ? N / 2 : 128, silu ? N / 2 : N, 0, 0, 0, status};
+  GemmParams p{(__half *)out, M, K, N, group, mt, silu ? N / 2 : 128, silu ? N / 2 : N, 0, 0, 0, status, early && pdl_enabled()};
   const bool in_tmem = mt <= GS_TMEM_MT;
   const int xb = mt * GS_BK * 2, w_cols = 512 - 2 * ((mt + 31) & ~31);
   p.dw = !in_tmem ? 3 : w_cols / GS_W_COLS < GS_MAX_DW ? w_cols / GS_W_COLS : GS_MAX_DW;
@@ -523,7 +524,7 @@ static int gemm_launch(const void *x, const int32_t *qweight, const void *scales
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  cfg.numAttrs = p.early ? 2 : 1;
   AB200_CUDA(cudaLaunchKernelEx(&cfg, kern, tm_x, tm_w, tm_s, p));
   return AB200_OK;
 }
@@ -537,11 +538,17 @@ extern "C" int ab200_w4a16_gemm(const void *x, const int32_t *qweight, const voi
   clear_error();
   AB200_REQUIRE(x && qweight && scales && out, "w4a16_gemm: null pointer");
   if (dtype != AB200_F16) return fail(AB200_EUNSUPPORTED, "w4a16_gemm: the tensor-core path is built for float16 (dtype %d given)", dtype);
-  return gemm_launch(x, qweight, scales, out, M, K, N, group, false, (cudaStream_t)stream);
+  return gemm_launch(x, qweight, scales, out, M, K, N, group, false, false, (cudaStream_t)stream);
+}
+
+extern "C" int ab200_w4a16_gemm_early(const void *x, const int32_t *qweight, const void *scales, void *out, int M, int K, int N, int group, int silu, void *stream) {
+  clear_error();
+  AB200_REQUIRE(!silu || N % 16 == 0, "w4a16_gemm_early: N=%d must be twice a multiple of 8", N);
+  return gemm_launch(x, qweight, scales, out, M, K, N, group, silu != 0, true, (cudaStream_t)stream);
 }
 
 extern "C" int ab200_w4a16_gemm_silu(const void *x, const int32_t *qweight, const void *scales, void *out, int M, int K, int N, int group, void *stream) {
   clear_error();
   AB200_REQUIRE(N % 16 == 0, "w4a16_gemm_silu: N=%d must be twice a multiple of 8", N);
-  return gemm_launch(x, qweight, scales, out, M, K, N, group, true, (cudaStream_t)stream);
+  return gemm_launch(x, qweight, scales, out, M, K, N, group, true, false, (cudaStream_t)stream);
 }

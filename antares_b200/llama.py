@@ -351,13 +351,16 @@ class LlamaInt4Decoder:
         cfg = self.cfg
         st = torch.cuda.current_stream().cuda_stream
         toks = self.prompt[:T]
+        for l in range(len(self.layers)):   # all made before the first launch below: the GEMMs read their weights early
+            for k in ("vqk", "o", "gu", "down"):
+                self._ref_layout(l, k)
         d, f = cfg.dim, self.fl
         x, xb, vqk, q, att, o, hh = b["x"], b["xb"], b["vqk"], b["q"], b["att"], b["o"], b["hh"]
         call("ab200_embed_rows", self.embed.data_ptr(), toks.data_ptr(), x.data_ptr(), T, d, cfg.vocab, st)
 
         def gemm(a, l, k, out):
             qw, sc = self._ref_layout(l, k)
-            call("ab200_w4a16_gemm", a.data_ptr(), qw.data_ptr(), sc.data_ptr(), out.data_ptr(), T, qw.shape[0] * 8, qw.shape[1], cfg.group, 0, st)
+            call("ab200_w4a16_gemm_early", a.data_ptr(), qw.data_ptr(), sc.data_ptr(), out.data_ptr(), T, qw.shape[0] * 8, qw.shape[1], cfg.group, 0, st)
 
         def residual(norm_w):
             """x += o, and the rows the next projection reads: their RMSNorm, in the same pass."""
@@ -386,7 +389,7 @@ class LlamaInt4Decoder:
             gemm(att, l, "o", o)
             residual(w["ffn_norm"])
             qw, sc = self._ref_layout(l, "gu")   # gate | up, silu(gate) * up on the way out
-            call("ab200_w4a16_gemm_silu", xb.data_ptr(), qw.data_ptr(), sc.data_ptr(), hh.data_ptr(), T, d, 2 * f, cfg.group, st)
+            call("ab200_w4a16_gemm_early", xb.data_ptr(), qw.data_ptr(), sc.data_ptr(), hh.data_ptr(), T, d, 2 * f, cfg.group, 1, st)
             gemm(hh, l, "down", o)
             residual(self.layers[l + 1]["att_norm"] if l + 1 < len(self.layers) else None)
         # classifier on the last token only, then the same bookkeeping as a decode step at pos = T - 1

@@ -172,6 +172,10 @@ int ab200_w4a16_gemm(const void *x, const int32_t *qweight, const void *scales, 
  * fp16-rounded projections, i.e. ab200_w4a16_gemm followed by ab200_silu_mul_rows in one pass. */
 int ab200_w4a16_gemm_silu(const void *x, const int32_t *qweight, const void *scales, void *out, int M,
                           int K, int N, int group, void *stream);
+/* Either of the two (silu 0 / 1), launched while the kernel before it in the stream still runs: the weights
+ * and scales are read at once and must date from before that kernel, x is not touched until it is done. */
+int ab200_w4a16_gemm_early(const void *x, const int32_t *qweight, const void *scales, void *out, int M,
+                           int K, int N, int group, int silu, void *stream);
 
 /* ---- elementwise / reduction operators ---------------------------------------------------- */
 

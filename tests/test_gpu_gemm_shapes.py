@@ -56,6 +56,9 @@ def test_prompt_gemm_with_swiglu(M, K, F, group):
     # silu's slope is at most 1.1; then one fp16 rounding and a few fp32 steps
     bound = 1.1 * dg * (u.abs() + du) + torch.nn.functional.silu(g).abs() * du + want.abs() * (2 ** -11 + 2 ** -20) + 2 ** -25
     assert bool(((out.double() - want).abs() <= bound).all())
+    early = torch.empty_like(out)
+    call("ab200_w4a16_gemm_early", x.data_ptr(), q.data_ptr(), s.data_ptr(), early.data_ptr(), M, K, 2 * F, group, 1, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(early, out)
     assert ops.kernel_status() == 0
 
 
