@@ -435,7 +435,8 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f16_kernel(GemvParams
 // The powers of two are exact: x is staged once as x * 2^e (2^e from the slice's largest magnitude, so that products
 // stay normal) times 2^(-4j), the zero-point leaves the loop as 8 * sum(x) per 32-k unit and the group scale is applied
 // per unit.  9 logic + 8 FFMA per packed word, against 8 shifts, 8 LOP3, 8 FADD, 8 FMUL, 8 FFMA when every nibble is
-// turned into scale * (q - 8) first.  A chain is the 8 k of one word, so that rounding errors stay below that form's.
+// turned into scale * (q - 8) first.  A chain is 4 k, so that rounding errors stay near that
+// form's although the nibbles are not centred.
 // A slice of x with an infinity or a NaN takes the plain form, whose special values are the operator's.
 // As in the fp16 kernel two units per warp are in flight in registers, the first before griddepcontrol.wait.
 template <int M>
@@ -562,10 +563,11 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f32_kernel(GemvParams
             t = fmaf(q[1], xa[m].y, t);
             t = fmaf(q[2], xa[m].z, t);
             t = fmaf(q[3], xa[m].w, t);
-            t = fmaf(q[4], xb[m].x, t);
-            t = fmaf(q[5], xb[m].y, t);
-            t = fmaf(q[6], xb[m].z, t);
-            acc[r][m][c] = fmaf(q[7], xb[m].w, t);
+            float v = q[4] * xb[m].x;
+            v = fmaf(q[5], xb[m].y, v);
+            v = fmaf(q[6], xb[m].z, v);
+            v = fmaf(q[7], xb[m].w, v);
+            acc[r][m][c] = t + v;
           }
         }
       }
