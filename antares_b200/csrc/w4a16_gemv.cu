@@ -429,19 +429,44 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f16_kernel(GemvParams
 // fp32 activations / scales / result: the dtypes the in-tree sample declares
 // (samples/05_llama2_7b_int4.py:75,133,139).
 //
-// Raw nibbles again, as fp32 bit patterns: a nibble left at bits 4j (j = 0..5) of a word is the number
-// q * 2^(4j - 149) - a subnormal, and for j = 5, whose top bit is the exponent's lowest, still linear in q - so
-// `w & (15 << 4j)` goes straight into an FFMA with x * 2^(e - 4j); the word shifted right by 8 gives the last two.
-// The powers of two are exact: x is staged once as x * 2^e (2^e from the slice's largest magnitude, so that products
-// stay normal) times 2^(-4j), the zero-point leaves the loop as 8 * sum(x) per 32-k unit and the group scale is applied
-// per unit.  9 logic + 8 FFMA per packed word, against 8 shifts, 8 LOP3, 8 FADD, 8 FMUL, 8 FFMA when every nibble is
-// turned into scale * (q - 8) first.  The nibbles are not centred, so a chain is 4 k and
-// sum(x) is taken in 64 bits: error against 64 bits over 24 drawn shapes 1.5e-7, 1.8e-7 for the plain form.  4096 x 12288 and
-// its like take 10.5 us a call on average, 16 in the plain form.
-// A slice of x with an infinity or a NaN takes the plain form, whose special values are the operator's.
+// The integer weight q - 8 is made without shifting every nibble down: `(w & 15 << 4j) | 0x4B000000` is the number
+// 2^23 + q * 16^j (j = 0..4), one subtraction leaves (q - 8) * 16^j exactly, and x was staged once as x * 16^(4 - j), a
+// power of two.  Nibbles 5..7 take the places 2..4 of `w >> 12`.  Products are centred, as the operator has them: nothing
+// has to cancel afterwards, whatever the size of an activation that meets a zero weight.  The group scale is applied
+// once per 32-k unit.  Pairs of k share the packed fp32 instructions: 1 shift + 8 logic + 4 + 4 per packed word,
+// against 8 shifts, 8 logic, 8 FADD, 8 FMUL, 8 FFMA when every nibble is turned into scale * (q - 8) first.
+// Products carry 2^16; a slice of x whose largest value is 2^103 or more (sums of 32 x * 8 * 2^16 could pass the top of
+// the range; infinities and NaN too) or below 2^-95 takes the plain form, and so does a unit whose scales are not finite:
+// special values are then the operator's.  Over 24 shapes (K 1024-11008, N 1448-21520, one row) the mean error against
+// 64 bits is 1.09e-7 and a call takes 15 us, the plain form 2.34e-7 (1.2e-7 at K = 1024) and 30 us; raw nibbles without
+// the subtraction (uncentred, the zero-point taken off as 8 * sum x) 1.54e-7 and 14.6 us, but an activation that meets zero
+// weights then leaves its rounding error behind, and sums from 2^120 on overflow.
 // As in the fp16 kernel two units per warp are in flight in registers, the first before griddepcontrol.wait.
+__device__ __forceinline__ uint64_t pack2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) { return pack2(__uint_as_float(lo), __uint_as_float(hi)); }
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ float sum2(uint64_t a) {
+  float lo, hi;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+  return lo + hi;
+}
+
+// One row: three CTAs an SM (80 registers), which the cluster sizes of pick_cluster count on.
 template <int M>
-__global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f32_kernel(GemvParams p) {
+__global__ void __launch_bounds__(GEMV_THREADS, M == 1 ? 3 : 2) w4a16_gemv_f32_kernel(GemvParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::cluster_group cluster = cg::this_cluster();
   const unsigned cs = cluster.num_blocks(), krank = cluster.block_rank();
@@ -450,13 +475,11 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f32_kernel(GemvParams
   const int n0 = tile * TILE_N + lane * 4, n0c = n0 < p.N ? n0 : p.N - 4;  // columns beyond N: read the last ones, never stored
   const int u_begin = (int)((long)p.units * krank / cs), u_end = (int)((long)p.units * (krank + 1) / cs);
   const int k_begin = u_begin * UNIT_K, kslice = (u_end - u_begin) * UNIT_K;
-  const int n_units = u_end - u_begin;
 
   const int xs_stride = p.xs_stride;
   float *xs = reinterpret_cast<float *>(smem_raw);
   float *red = xs + (size_t)M * xs_stride;
   float *part = red + GEMV_WARPS * M * TILE_N;
-  float *corr = part + M * TILE_N;  // [M][units of the slice]: 8 * sum over the unit of x
   __shared__ unsigned sh_max[M][GEMV_WARPS];
 
   constexpr int NBUF = 2;
@@ -480,104 +503,75 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f32_kernel(GemvParams
     if (u_load < u_end) load_unit(b);
   pdl_wait();  // x (and the output buffer) may come from the kernel before this one
 
-  // stage x; per batch row the largest magnitude of the slice
+  // stage x times 16^(4 - j), j the place of k: 0 1 2 3 | 4 2 3 4 (a quad is one half of a packed row); per batch row the
+  // largest magnitude of the slice
   const float *xg = reinterpret_cast<const float *>(p.x);
   const int quads = kslice / 4;
-  unsigned mx[M];
 #pragma unroll
   for (int m = 0; m < M; ++m) {
-    mx[m] = 0u;
+    unsigned mx = 0u;
     for (int i = threadIdx.x; i < quads; i += GEMV_THREADS) {
-      const uint4 v = *reinterpret_cast<const uint4 *>(xg + (size_t)m * p.K + k_begin + i * 4);
-      *reinterpret_cast<uint4 *>(xs + (size_t)m * xs_stride + i * 4) = v;
-      mx[m] = max(mx[m], max(max(v.x & 0x7FFFFFFFu, v.y & 0x7FFFFFFFu), max(v.z & 0x7FFFFFFFu, v.w & 0x7FFFFFFFu)));
+      const float4 v = *reinterpret_cast<const float4 *>(xg + (size_t)m * p.K + k_begin + i * 4);
+      *reinterpret_cast<float4 *>(xs + (size_t)m * xs_stride + i * 4) =
+          (i & 1) ? make_float4(v.x, v.y * 0x1p8f, v.z * 0x1p4f, v.w) : make_float4(v.x * 0x1p16f, v.y * 0x1p12f, v.z * 0x1p8f, v.w * 0x1p4f);
+      mx = max(mx, max(max(__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.y) & 0x7FFFFFFFu),
+                       max(__float_as_uint(v.z) & 0x7FFFFFFFu, __float_as_uint(v.w) & 0x7FFFFFFFu)));
     }
-    mx[m] = __reduce_max_sync(0xffffffffu, mx[m]);
-    if (lane == 0) sh_max[m][warp] = mx[m];
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if (lane == 0) sh_max[m][warp] = mx;
   }
   __syncthreads();
   bool plain = false;
-  float back1[M], back2[M];  // 2^(149 - e) as two factors
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     unsigned t = 0u;
 #pragma unroll
     for (int w = 0; w < GEMV_WARPS; ++w) t = max(t, sh_max[m][w]);
-    const int E = max((int)(t >> 23), 1);  // biased exponent: |x| < 2^(E - 126)
-    plain = plain || E == 255;
-    // |x| * 2^e < 2^120, products below 15 * 2^-29; e is 246 - E as two exact factors
-    const int e = 246 - E, e1 = e / 2, e2 = e - e1;
-    const float f1 = __int_as_float((127 + e1) << 23), f2 = __int_as_float((127 + e2) << 23);
-    const int b1 = (149 - e) / 2, b2 = 149 - e - b1;
-    back1[m] = __int_as_float((127 + b1) << 23);
-    back2[m] = __int_as_float((127 + b2) << 23);
-    // second pass over the same elements: x * 2^e * 2^(-4j) with j = 0 .. 5, 4, 5 for k = 0 .. 7, and the unit sums
-    // (two quads = one packed row; eight adjacent lanes = one unit)
-    if (E != 255) {
-      const int pad = (quads + 31) & ~31;
-      for (int i = threadIdx.x; i < pad; i += GEMV_THREADS) {
-        double sx = 0.0;  // in 64 bits: its rounding would be every column's error
-        if (i < quads) {
-          float4 *slot = reinterpret_cast<float4 *>(xs + (size_t)m * xs_stride + i * 4);
-          const float4 v = *slot;
-          sx = ((double)v.x + v.y) + ((double)v.z + v.w);
-          const float4 w = make_float4(v.x * f1 * f2, v.y * f1 * f2, v.z * f1 * f2, v.w * f1 * f2);
-          *slot = (i & 1) ? make_float4(w.x * 0x1p-16f, w.y * 0x1p-20f, w.z * 0x1p-16f, w.w * 0x1p-20f)
-                          : make_float4(w.x, w.y * 0x1p-4f, w.z * 0x1p-8f, w.w * 0x1p-12f);
-        }
-        sx += __shfl_xor_sync(0xffffffffu, sx, 1);
-        sx += __shfl_xor_sync(0xffffffffu, sx, 2);
-        sx += __shfl_xor_sync(0xffffffffu, sx, 4);
-        if (i < quads && (i & 7) == 0) corr[m * n_units + (i >> 3)] = (float)(8.0 * sx);
-      }
-    }
+    plain = plain || t >= 0x73000000u || (t != 0u && t < 0x10000000u);  // 2^103, 2^-95
   }
-  __syncthreads();
 
   float facc[M][4];
 #pragma unroll
   for (int m = 0; m < M; ++m)
 #pragma unroll
     for (int c = 0; c < 4; ++c) facc[m][c] = 0.f;
+  constexpr uint32_t MAGIC = 0x4B000000u;  // 2^23
+  const uint64_t c01 = pack2(-8388616.f, -8388736.f), c23 = pack2(-8390656.f, -8421376.f), c42 = pack2(-8912896.f, -8390656.f),
+                 c34 = pack2(-8421376.f, -8912896.f);  // -(2^23 + 8 * 16^j) for the places 0 1, 2 3, 4 2, 3 4
   auto compute_unit = [&](int b) {
     const float sc[4] = {sbuf[b].x, sbuf[b].y, sbuf[b].z, sbuf[b].w};
     const float *xu = xs + (u - u_begin) * UNIT_K;
-    if (!plain) {
-      float acc[UNIT_ROWS][M][4];
+    if (!plain && fmaf(sc[0], 0.f, fmaf(sc[1], 0.f, fmaf(sc[2], 0.f, sc[3] * 0.f))) == 0.f) {
+      uint64_t acc[2][M][4];  // even and odd packed rows
 #pragma unroll
       for (int r = 0; r < UNIT_ROWS; ++r) {
-        float4 xa[M], xb[M];
+        ulonglong2 xa[M], xb[M];
 #pragma unroll
         for (int m = 0; m < M; ++m) {
-          xa[m] = *reinterpret_cast<const float4 *>(xu + (size_t)m * xs_stride + r * 8);
-          xb[m] = *reinterpret_cast<const float4 *>(xu + (size_t)m * xs_stride + r * 8 + 4);
+          xa[m] = *reinterpret_cast<const ulonglong2 *>(xu + (size_t)m * xs_stride + r * 8);
+          xb[m] = *reinterpret_cast<const ulonglong2 *>(xu + (size_t)m * xs_stride + r * 8 + 4);
         }
         const uint32_t wr[4] = {wbuf[b][r].x, wbuf[b][r].y, wbuf[b][r].z, wbuf[b][r].w};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
-          const uint32_t w = wr[c], w8 = w >> 8;
-          const float q[8] = {__uint_as_float(w & 0xFu),       __uint_as_float(w & 0xF0u),     __uint_as_float(w & 0xF00u),    __uint_as_float(w & 0xF000u),
-                              __uint_as_float(w & 0xF0000u),   __uint_as_float(w & 0xF00000u), __uint_as_float(w8 & 0xF0000u), __uint_as_float(w8 & 0xF00000u)};
+          const uint32_t w = wr[c], v = w >> 12;
+          const uint64_t q01 = add2(pack2(lop3<0xEA>(w, 0xFu, MAGIC), lop3<0xEA>(w, 0xF0u, MAGIC)), c01);
+          const uint64_t q23 = add2(pack2(lop3<0xEA>(w, 0xF00u, MAGIC), lop3<0xEA>(w, 0xF000u, MAGIC)), c23);
+          const uint64_t q45 = add2(pack2(lop3<0xEA>(w, 0xF0000u, MAGIC), lop3<0xEA>(v, 0xF00u, MAGIC)), c42);
+          const uint64_t q67 = add2(pack2(lop3<0xEA>(v, 0xF000u, MAGIC), lop3<0xEA>(v, 0xF0000u, MAGIC)), c34);
 #pragma unroll
           for (int m = 0; m < M; ++m) {
-            float t = q[0] * xa[m].x;
-            t = fmaf(q[1], xa[m].y, t);
-            t = fmaf(q[2], xa[m].z, t);
-            t = fmaf(q[3], xa[m].w, t);
-            float v = q[4] * xb[m].x;
-            v = fmaf(q[5], xb[m].y, v);
-            v = fmaf(q[6], xb[m].z, v);
-            v = fmaf(q[7], xb[m].w, v);
-            acc[r][m][c] = t + v;
+            uint64_t t = fma2(q01, xa[m].x, r < 2 ? 0ull : acc[r & 1][m][c]);
+            t = fma2(q23, xa[m].y, t);
+            t = fma2(q45, xb[m].x, t);
+            acc[r & 1][m][c] = fma2(q67, xb[m].y, t);
           }
         }
       }
 #pragma unroll
-      for (int m = 0; m < M; ++m) {
-        const float zp = corr[m * n_units + (u - u_begin)];
+      for (int m = 0; m < M; ++m)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) facc[m][c] = fmaf(sc[c], fmaf(((acc[0][m][c] + acc[1][m][c]) + (acc[2][m][c] + acc[3][m][c])) * back1[m], back2[m], -zp), facc[m][c]);
-      }
+        for (int c = 0; c < 4; ++c) facc[m][c] = fmaf(sc[c], sum2(add2(acc[0][m][c], acc[1][m][c])) * 0x1p-16f, facc[m][c]);
     } else {
 #pragma unroll 1
       for (int r = 0; r < UNIT_ROWS; ++r) {
