@@ -441,7 +441,8 @@ __global__ void __launch_bounds__(GEMV_THREADS) w4a16_gemv_f16_kernel(GemvParams
 // 64 bits is 1.09e-7 and a call takes 15 us, the plain form 2.34e-7 (1.2e-7 at K = 1024) and 30 us; raw nibbles without
 // the subtraction (uncentred, the zero-point taken off as 8 * sum x) 1.54e-7 and 14.6 us, but an activation that meets zero
 // weights then leaves its rounding error behind, and sums from 2^120 on overflow.
-// As in the fp16 kernel two units per warp are in flight in registers, the first before griddepcontrol.wait.
+// As in the fp16 kernel two units per warp are in flight in registers; unlike there nothing is read before
+// griddepcontrol.wait.
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
@@ -498,10 +499,10 @@ __global__ void __launch_bounds__(GEMV_THREADS, M == 1 ? 3 : 2) w4a16_gemv_f32_k
   };
   if (cs > 1) cluster_arrive_started();
   pdl_launch_dependents();
+  pdl_wait();  // everything may come from the kernel before this one: callers convert scales to fp32 right before the call
 #pragma unroll
   for (int b = 0; b < NBUF; ++b)
     if (u_load < u_end) load_unit(b);
-  pdl_wait();  // x (and the output buffer) may come from the kernel before this one
 
   // stage x times 16^(4 - j), j the place of k: 0 1 2 3 | 4 2 3 4 (a quad is one half of a packed row); per batch row the
   // largest magnitude of the slice

@@ -82,3 +82,16 @@ def test_f32_gemv_scales_that_are_not_finite(value):
     nib, sw = _wide(q, s, 128)
     want = x.double() @ ((nib - 8) * sw)
     assert bool(want[0, 10].isnan()) and bool(y[0, 10].isnan()) and int(y.isfinite().sum()) == 255
+
+
+@pytest.mark.parametrize("K,N", [(4096, 256), (11008, 4096)])
+def test_f32_gemv_scales_from_the_kernel_before(K, N):
+    """The scales of a call are the result of the one launched just before it, which lets its successor start early."""
+    x, q, s = _case(1, K, N, 128, 11)
+    x2, q2, _ = _case(1, 128, N, 128, 12)
+    want = ops.w4a16_gemv(x, q, s).clone()
+    torch.cuda.synchronize()
+    ref = ops.w4a16_gemv(x2, q2, want.view(1, N))
+    torch.cuda.synchronize()
+    for _ in range(20):
+        assert torch.equal(ops.w4a16_gemv(x2, q2, ops.w4a16_gemv(x, q, s).view(1, N)), ref)
