@@ -76,6 +76,16 @@ def _split_call(match, tensors, out):
     return by_name, out
 
 
+def _settle(given, used):
+    """Called before a W4A16 launch with the weights a caller gave and those the launch reads.  The fp16 decode kernels bring
+    weights and scales in before they wait for the kernel ahead of them, so that one must not be the copy that made them
+    contiguous: a fill in between does not start before the copy is complete and visible."""
+    for a, b in zip(given, used):
+        if a is not b and b.is_cuda:
+            torch.zeros(1, device=b.device)
+            return
+
+
 class NativeModules:
     """Keys of the library's native plugin boundary (ab200_inject / ab200_forward, the counterpart of
     frameworks/pytorch/main_ops.cc:17-54) for one exported op: the kernel-source text is written in the
@@ -151,6 +161,7 @@ def export(ir, inputs, config=None, name=None):
             if match.kind == "w4a16":
                 qw = t[pr["qweight"]]
                 shape = tuple(x.shape[:-1]) + (qw.shape[1],)
+                _settle(*zip(*((a, b) for n, a, b in zip(names, tensors, ordered) if n != pr["x"])))
             else:
                 shape = tuple(x.shape)
             if out is None:

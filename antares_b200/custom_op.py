@@ -60,6 +60,9 @@ class CustomOp(torch.nn.Module):
             shape = tuple(x.shape[:-1]) + (t[pr["qweight"]].shape[1],) if self.match.kind == "w4a16" else tuple(x.shape)
             out = torch.empty(shape, dtype=x.dtype, device=x.device)
             dt = {torch.float16: "float16", torch.float32: "float32"}[x.dtype]
+            if self.match.kind == "w4a16":
+                from .autort_api import _settle
+                _settle(*zip(*((a, t[k]) for k, a in zip(self.input_names, inputs) if k != pr["x"])))
             return self.native.forward([t[s.name] for s in self.match.inputs], out, dt)
         if self.match.kind == "eltwise":
             ins = [t[n] for n in pr["inputs"]]

@@ -90,7 +90,10 @@ int ab200_w4_dequant(const int32_t *qweight, const void *scales, int K, int N, i
  * the exported op `my_custom_fn` of samples/05_llama2_7b_int4.py:135-144 (`matmul_dequat`).
  * This is the decode path (M <= 16): weights are streamed once from HBM.
  * Constraints: K % 32 == 0, group % 32 == 0, K % group == 0, N % 4 == 0, 1 <= M <= 16,
- * pointers 16-byte aligned. */
+ * pointers 16-byte aligned.
+ * fp16, this and every fp16 entry below: qweight and scales are read while the kernel before it in the
+ * stream may still run (option "pdl"), so they must date from before that kernel; x and out need not.
+ * The fp32 form reads nothing before that kernel is complete. */
 int ab200_w4a16_gemv(const void *x, const int32_t *qweight, const void *scales, void *out, int M,
                      int K, int N, int group, int dtype, void *stream);
 

@@ -211,3 +211,29 @@ def test_layernorm_ir_runs_on_the_row_reduction_template(cuda):
     assert yh.dtype == torch.float16 and _err(yh.cpu().numpy(), want2) <= 1e-2
     # bitwise repeatable (fixed reduction order)
     assert torch.equal(op(torch.from_numpy(xh), torch.from_numpy(g), torch.from_numpy(b)), yh)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+def test_weights_that_the_call_has_to_copy(cuda, dtype, monkeypatch):
+    """Strided weights and scales are copied by the call itself: the result is that of the contiguous ones, whatever the copies'
+    memory held before, and something stands between the copy and a launch that may read its weights early."""
+    from antares_b200 import autort_api
+    fills = []
+    zeros = torch.zeros
+    monkeypatch.setattr(autort_api.torch, "zeros", lambda *a, **k: fills.append(a) or zeros(*a, **k))
+    name = {torch.float16: "float16", torch.float32: "float32"}[dtype]
+    fn = autort.export(ir=W4A16_IR, inputs=["input0=%s[S:4096]" % name, "qweight=int32[L:512, N:4096]", "scales=%s[K:32, N:4096]" % name], name="copied_" + name)
+    op = CustomOp(ir=W4A16_IR, input_orders={"input0": ([], dtype, [4096]), "qweight": ([], torch.int32, [512, 2048]), "scales": ([], dtype, [32, 2048])}).tune().emit()
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(4096, generator=g, device="cuda").to(dtype)
+    for i in range(8):
+        q = torch.randint(-2 ** 31, 2 ** 31, (512, 4096), generator=g, device="cuda", dtype=torch.int32)
+        s = (torch.rand(32, 4096, generator=g, device="cuda") * 0.02).to(dtype)
+        want = fn(x, q[:, :2048].contiguous(), s[:, :2048].contiguous())
+        torch.cuda.synchronize()
+        n = len(fills)
+        for f in (fn, op):
+            assert torch.equal(f(x, q[:, :2048], s[:, :2048]), want)
+        assert len(fills) == n + 2
+        fn(torch.stack([x, x], 1)[:, 0], q[:, :2048].contiguous(), s[:, :2048].contiguous())
+        assert len(fills) == n + 2
