@@ -188,7 +188,8 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
   while (threads < RV_MAX_THREADS && threads * VM_E < cols) threads *= 2;
   const int cap = sm_count() * (2048 / threads);
   const size_t smem = (size_t)stack * threads * VM_E * sizeof(float);
-  if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(rowreduce_vm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // the limit that needs no opting in, 48 KiB, is on this and the static arrays (under 2 KiB) together
+  if (smem > 46 * 1024) AB200_CUDA(cudaFuncSetAttribute(rowreduce_vm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   rowreduce_vm_kernel<<<rows < cap ? rows : cap, threads, smem, (cudaStream_t)stream>>>(p);
   AB200_CHECK_LAUNCH("rowreduce_vm");
   return AB200_OK;

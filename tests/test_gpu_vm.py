@@ -59,3 +59,19 @@ def test_row_programs_at_odd_sizes(rows, cols, dtype):
     flat = torch.zeros(rows * cols + 1, dtype=dt, device="cuda")[1:].view(rows, cols)  # unaligned input
     flat.copy_(x)
     np.testing.assert_allclose(fn(flat, w, c).float().cpu().numpy(), want, rtol=tol, atol=tol * max(1e-3, np.abs(want).max()))
+
+
+@pytest.mark.parametrize("depth", [3, 5, 6])
+@pytest.mark.parametrize("cols", [1000, 1025, 2050])
+def test_row_programs_with_deep_expressions(depth, cols):
+    """The operand stack is shared memory, up to 48 KiB of it in the widest block."""
+    expr = "x[N, C] + %d.0" % (depth + 1)
+    for i in range(depth, 0, -1):
+        expr = "(x[N, C] + %d.0) * (%s)" % (i, expr)
+    text = "s[N] +=! x[N, C]; y[N, C] = %s - s[N]" % expr
+    fn = autort.export(ir=text, inputs=["x=float32[N:8, C:4096]"], name="deep_%d" % depth)
+    x = torch.randn(3, cols, generator=torch.Generator(device="cuda").manual_seed(cols), device="cuda")
+    rp = fn.match.params
+    want = eval_row_program_numpy(rp, [x.cpu().numpy()], [])
+    # sums of up to 2050 terms in another order, products of up to 7 factors of 2^-24 each
+    np.testing.assert_allclose(fn(x).cpu().numpy(), want, rtol=2e-5, atol=2e-5 * np.abs(want).max())
