@@ -25,7 +25,7 @@
 //
 // Values of V that are not finite: a masked or underflowed probability is exactly 0 in the MMA, and 0 * inf
 // would reach rows that never attend to that key.  The loading warps look at every V tile; a CTA that saw one
-// recomputes its rows with fp32 code that touches only the keys a row attends to (attend_row below).
+// recomputes its rows with fp32 code that touches only the keys a row attends to (attend_rows below).
 #include <math_constants.h>
 
 #include <type_traits>
@@ -122,33 +122,103 @@ __device__ __forceinline__ float ap_ex2(float x) {
   return y;
 }
 
-// One query row by one warp in fp32, two passes over exactly the keys it attends to (lane = 4 dims).
-__device__ __noinline__ void attend_row(const AttnPrefillParams &p, int h, int row, int S) {
-  const int lane = threadIdx.x & 31;
-  const size_t at = ((size_t)row * p.H + h) * AP_D + lane * 4;
-  auto ld4 = [](const __half *s, float (&f)[4]) {
-    const uint2 v = *reinterpret_cast<const uint2 *>(s);
+// Four consecutive query rows by one warp in fp32, two passes over exactly the keys each attends to (lane = 4 dims).
+// Four keys at a time: their rows are loaded once for the four queries, and the 16 dot products are summed over the warp
+// together (16 shuffles), lane 2 i + (0, 1) ending with the score of key i / 4 and row i % 4.
+// 32 heads with a value that is not finite, us: 70 / 128 / 512 / 2000 rows 83 / 147 / 639 / 4170; the single-query kernel once
+// per row 24 / 42 / 306 / 4020; a warp with one row and one key at a time 2574 at 128 rows, 47242 at 2000.
+__device__ __noinline__ void attend_rows(const AttnPrefillParams &p, int h, int row0, int pos0) {
+  constexpr int R = 4, KEYS = 4;
+  const int lane = threadIdx.x & 31, my_key = lane >> 3, my_row = (lane >> 1) & 3;
+  auto wide4 = [](uint2 v, float (&f)[4]) {
     const float2 a = __half22float2(u2h2(v.x)), b = __half22float2(u2h2(v.y));
     f[0] = a.x, f[1] = a.y, f[2] = b.x, f[3] = b.y;
   };
-  float qf[4], f[4];
-  ld4(p.q + at, qf);
-  auto score = [&](int s) {
-    ld4(p.kc + kv_row(p.pages, s) * p.kv_stride + (size_t)h * AP_D + lane * 4, f);
-    return warp_sum(qf[0] * f[0] + qf[1] * f[1] + qf[2] * f[2] + qf[3] * f[3]) * p.scale;
+  auto limit = [&](int r) {  // cache rows that row row0 + r attends to; not falling with r
+    const long s = (long)pos0 + 1 + min(row0 + r, p.rows - 1);
+    return (int)(s < 0 ? 0 : s > p.max_seq ? p.max_seq : s);
   };
-  float mx = -CUDART_INF_F, l = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int s = 0; s < S; ++s) mx = fmaxf(mx, score(s));
-  for (int s = 0; s < S; ++s) {
-    const float e = expf(score(s) - mx);
-    l += e;
-    ld4(p.vc + kv_row(p.pages, s) * p.kv_stride + (size_t)h * AP_D + lane * 4, f);
+  float qf[R][4], acc[R][4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = fmaf(e, f[j], acc[j]);
+  for (int r = 0; r < R; ++r) {
+    wide4(*reinterpret_cast<const uint2 *>(p.q + ((size_t)min(row0 + r, p.rows - 1) * p.H + h) * AP_D + lane * 4), qf[r]);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[r][j] = 0.f;
   }
-  __half *o = p.out + at;
+  const int S = limit(R - 1), S_mine = limit(my_row);
+  const size_t at = (size_t)h * AP_D + lane * 4;
+  // the four keys from s0 on are asked for while the four before them are worked on; beyond the last one in use: that one again
+  auto ask = [&](const __half *base, int s0, uint2 (&v)[KEYS]) {
 #pragma unroll
-  for (int j = 0; j < 4; ++j) o[j] = __float2half_rn(S > 0 ? acc[j] / l : 0.f);
+    for (int k = 0; k < KEYS; ++k) v[k] = *reinterpret_cast<const uint2 *>(base + kv_row(p.pages, min(s0 + k, S - 1)) * p.kv_stride + at);
+  };
+  auto score = [&](const uint2 (&v)[KEYS]) {
+    float f[KEYS][4], d[KEYS * R];
+#pragma unroll
+    for (int k = 0; k < KEYS; ++k) wide4(v[k], f[k]);
+#pragma unroll
+    for (int i = 0; i < KEYS * R; ++i) {
+      const float(&x)[4] = qf[i % R];
+      const float(&y)[4] = f[i / R];
+      d[i] = x[0] * y[0] + x[1] * y[1] + x[2] * y[2] + x[3] * y[3];
+    }
+#pragma unroll
+    for (int n = KEYS * R / 2, o = 16; n >= 1; n >>= 1, o >>= 1)
+#pragma unroll
+      for (int i = 0; i < n; ++i) {
+        const float keep = lane & o ? d[i + n] : d[i], send = lane & o ? d[i] : d[i + n];
+        d[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
+    return (d[0] + __shfl_xor_sync(0xffffffffu, d[0], 1)) * p.scale;
+  };
+  float mx = -CUDART_INF_F, l = 0.f;
+  uint2 k_now[KEYS], k_next[KEYS], v_now[KEYS], v_next[KEYS];
+  if (S > 0) ask(p.kc, 0, k_next);
+  for (int s0 = 0; s0 < S; s0 += KEYS) {
+#pragma unroll
+    for (int k = 0; k < KEYS; ++k) k_now[k] = k_next[k];
+    ask(p.kc, s0 + KEYS, k_next);
+    const float t = score(k_now);
+    mx = s0 + my_key < S_mine ? fmaxf(mx, t) : mx;
+  }
+#pragma unroll
+  for (int o = 8; o <= 16; o <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (S > 0) ask(p.kc, 0, k_next), ask(p.vc, 0, v_next);
+  for (int s0 = 0; s0 < S; s0 += KEYS) {
+#pragma unroll
+    for (int k = 0; k < KEYS; ++k) k_now[k] = k_next[k], v_now[k] = v_next[k];
+    ask(p.kc, s0 + KEYS, k_next);
+    ask(p.vc, s0 + KEYS, v_next);
+    const float e = expf(score(k_now) - mx);
+    l += s0 + my_key < S_mine ? e : 0.f;
+    float f[KEYS][4];
+#pragma unroll
+    for (int k = 0; k < KEYS; ++k) wide4(v_now[k], f[k]);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int S_r = __shfl_sync(0xffffffffu, S_mine, 2 * r);
+#pragma unroll
+      for (int k = 0; k < KEYS; ++k) {
+        const float er = __shfl_sync(0xffffffffu, e, 8 * k + 2 * r);
+        if (s0 + k < S_r) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[r][j] = fmaf(er, f[k][j], acc[r][j]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 8; o <= 16; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const float lr = __shfl_sync(0xffffffffu, l, 2 * r);
+    const int S_r = __shfl_sync(0xffffffffu, S_mine, 2 * r);
+    if (row0 + r < p.rows) {
+      __half *o = p.out + (size_t)(row0 + r) * p.H * AP_D + at;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) o[j] = __float2half_rn(S_r > 0 ? acc[r][j] / lr : 0.f);
+    }
+  }
 }
 
 __global__ void __launch_bounds__(AP_THREADS, 2) attention_prefill_kernel(AttnPrefillParams p) {
@@ -421,25 +491,24 @@ __global__ void __launch_bounds__(AP_THREADS, 2) attention_prefill_kernel(AttnPr
 #pragma unroll
         for (int i = 0; i < 16; ++i) *reinterpret_cast<uint4 *>(park + lane * AP_ROWB + i * 16) = make_uint4(0, 0, 0, 0);
       }
-      __syncwarp();
-      const int piece = lane & 15;
-#pragma unroll 4
-      for (int rr = 0; rr < 32; rr += 2) {
-        const int rl = rr + (lane >> 4), row = q0 + warp * 32 + rl;
-        const uint4 v = *reinterpret_cast<const uint4 *>(park + rl * AP_ROWB + piece * 16);
-        if (row < p.rows) *reinterpret_cast<uint4 *>(p.out + ((size_t)row * p.H + h) * AP_D + piece * 8) = v;
-      }
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == AP_MMA_WARP) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "n"(AP_TMEM_COLS) : "memory");
+  // Nothing is stored before it is known which of the two results it is: `out` may be `q`, which the other one reads again.
   if (fail_s) {
     if (tid == 0) atomicExch(p.status, 700);  // site 700: a wait of the prompt attention ran out
-  } else if (bad_s && warp < AP_SOFT_WARPS) {
-    for (int r = 0; r < 32; ++r) {
-      const int row = q0 + warp * 32 + r;
-      if (row < p.rows) attend_row(p, h, row, limit_of(row));
+  } else if (bad_s) {
+    for (int r = warp * 4; r < AP_BM && q0 + r < p.rows; r += AP_THREADS / 32 * 4) attend_rows(p, h, q0 + r, pos0);
+  } else if (warp < AP_SOFT_WARPS) {
+    const unsigned char *park = smem + (size_t)warp * 32 * AP_ROWB;
+    const int piece = lane & 15;
+#pragma unroll 4
+    for (int rr = 0; rr < 32; rr += 2) {
+      const int rl = rr + (lane >> 4), row = q0 + warp * 32 + rl;
+      const uint4 v = *reinterpret_cast<const uint4 *>(park + rl * AP_ROWB + piece * 16);
+      if (row < p.rows) *reinterpret_cast<uint4 *>(p.out + ((size_t)row * p.H + h) * AP_D + piece * 8) = v;
     }
   }
 }

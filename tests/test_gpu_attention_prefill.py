@@ -12,9 +12,10 @@ pytestmark = pytest.mark.gpu
 H, D = 3, 128
 
 
-def _run(q, k, v, pos0, scale, table=None, page_rows=0, max_seq=None):
+def _run(q, k, v, pos0, scale, table=None, page_rows=0, max_seq=None, in_place=False):
     rows, max_seq = q.shape[0], max_seq or k.shape[0]
-    out = torch.full_like(q, 7.0)
+    q = q.clone() if in_place else q
+    out = q if in_place else torch.full_like(q, 7.0)
     pos = torch.tensor([pos0], dtype=torch.int32, device="cuda")
     args = [q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), pos.data_ptr(), rows, max_seq, H, D, k.stride(0), scale]
     if table is None:
@@ -93,3 +94,19 @@ def test_values_that_are_not_finite_reach_only_the_rows_that_attend(value, at):
     fine = want.isfinite()
     _close(got[fine], want[fine], v[:rows][v[:rows].isfinite()])
     assert torch.equal(fine[:at], torch.ones_like(fine[:at]))
+
+
+@pytest.mark.parametrize("rows", [5, 70, 300])
+@pytest.mark.parametrize("value", [1.0, math.inf, math.nan])
+def test_result_over_the_queries(rows, value):
+    """`out` may be `q`: a row's query is read before its result is stored, whichever code computes it."""
+    q, k, v = _inputs(rows, 320, rows)
+    v[3, 5] = value
+    got = _run(q, k, v, 0, 0.09, in_place=True)
+    want = _run(q, k, v, 0, 0.09)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[~got.isnan()], want[~want.isnan()])
+    _close(got[want.isfinite()], _expected(q, k, v, 0, 0.09)[want.isfinite()], v[:rows][v[:rows].isfinite()])
+    # the page table form, and every row in a tile whose values are not finite
+    table = torch.arange(80, device="cuda", dtype=torch.int32)
+    paged = _run(q, k, v, 0, 0.09, table, 4, 320, in_place=True)
+    assert torch.equal(paged.isnan(), want.isnan()) and torch.equal(paged[~want.isnan()], want[~want.isnan()])
