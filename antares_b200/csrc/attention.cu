@@ -40,7 +40,9 @@ __device__ __forceinline__ void h8_to_f8(const uint4 v, float (&f)[8]) {
 // samples/05_llama2_7b_int4.py:161-165): p = softmax_s(scale * q.K_s), out = sum_s p_s V_s.
 // Phase 1: a half-warp per cache row computes the score (16 lanes x 8 dims).
 // Phase 2: block-wide max / sum of exp.  Phase 3: 16 row-groups x 16 dim-chunks accumulate P.V.
-template <typename T>
+// AT: the number of rows is seq_len_add alone and the scale is on the device.  (As run-time choices the two cost the
+// other form its register allocation: 40 rows of 32 heads behind 500 cached rows 56 us, so 51.)
+template <typename T, bool AT>
 __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(const T *__restrict__ q, const T *__restrict__ kc,
                                                                       const T *__restrict__ vc, T *__restrict__ out,
                                                                       const int32_t *__restrict__ seq_len_dev, int seq_len_add,
@@ -52,8 +54,8 @@ __global__ void __launch_bounds__(ATT_THREADS) attention_decode_kernel(const T *
   __shared__ float sh[32];
   const int h = blockIdx.x;
   // blockIdx.y = query row of a causal prefill: row r sees r more cache rows than row 0
-  int S = (seq_len_dev ? *seq_len_dev : 0) + seq_len_add + (int)blockIdx.y;
-  if (scale_dev) scale = *scale_dev;
+  int S = (AT ? 0 : *seq_len_dev) + seq_len_add + (int)blockIdx.y;
+  if (AT) scale = *scale_dev;
   S = S < 0 ? 0 : (S > max_seq ? max_seq : S);
   q += (size_t)blockIdx.y * gridDim.x * ATT_D;
   out += (size_t)blockIdx.y * gridDim.x * ATT_D;
@@ -357,21 +359,18 @@ static int attention_decode_impl(const void *q_f16, const void *k_cache_f16, con
                 "attention_decode: pointers must be 16-byte aligned");
   const size_t smem = ((size_t)max_seq + 16 * ATT_D) * sizeof(float);
   if (smem > 200 * 1024) return fail(AB200_EUNSUPPORTED, "attention_decode: max_seq=%d exceeds the shared-memory score buffer", max_seq);
-  if (dtype == AB200_F16) {
-    if (smem > 48 * 1024)
-      AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attention_decode_kernel<__half><<<H, ATT_THREADS, smem, (cudaStream_t)stream>>>((const __half *)q_f16, (const __half *)k_cache_f16,
-                                                                                   (const __half *)v_cache_f16, (__half *)out_f16, seq_len_dev,
-                                                                                   seq_len_add, max_seq, kv_stride, scale, scale_dev, KvPages{nullptr, 0});
-  } else if (dtype == AB200_F32) {
-    if (smem > 48 * 1024)
-      AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    attention_decode_kernel<float><<<H, ATT_THREADS, smem, (cudaStream_t)stream>>>((const float *)q_f16, (const float *)k_cache_f16,
-                                                                                  (const float *)v_cache_f16, (float *)out_f16, seq_len_dev,
-                                                                                  seq_len_add, max_seq, kv_stride, scale, scale_dev, KvPages{nullptr, 0});
-  } else {
-    return fail(AB200_EINVAL, "attention_decode: unknown dtype %d", dtype);
-  }
+  auto launch = [&](auto kern, auto elt) -> int {
+    using T = decltype(elt);
+    if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    kern<<<H, ATT_THREADS, smem, (cudaStream_t)stream>>>((const T *)q_f16, (const T *)k_cache_f16, (const T *)v_cache_f16, (T *)out_f16, seq_len_dev, seq_len_add,
+                                                         max_seq, kv_stride, scale, scale_dev, KvPages{nullptr, 0});
+    return AB200_OK;
+  };
+  int rc;
+  if (dtype == AB200_F16) rc = scale_dev ? launch(attention_decode_kernel<__half, true>, __half()) : launch(attention_decode_kernel<__half, false>, __half());
+  else if (dtype == AB200_F32) rc = scale_dev ? launch(attention_decode_kernel<float, true>, 0.f) : launch(attention_decode_kernel<float, false>, 0.f);
+  else return fail(AB200_EINVAL, "attention_decode: unknown dtype %d", dtype);
+  if (rc) return rc;
   AB200_CHECK_LAUNCH("attention_decode");
   return AB200_OK;
 }
@@ -478,8 +477,8 @@ static int attention_prefill_impl(const void *q_f16, const void *k_cache_f16, co
   if (rows >= ATT_PREFILL_TC_ROWS)
     return attention_prefill_launch(q_f16, k_cache_f16, v_cache_f16, out_f16, pos0_dev, rows, max_seq, H, kv_stride, scale,
                                     KvPages{page_table, page_table ? page_shift_of(page_rows) : 0}, (cudaStream_t)stream);
-  if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-  attention_decode_kernel<__half><<<dim3(H, rows), ATT_THREADS, smem, (cudaStream_t)stream>>>(
+  if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<__half, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+  attention_decode_kernel<__half, false><<<dim3(H, rows), ATT_THREADS, smem, (cudaStream_t)stream>>>(
       (const __half *)q_f16, (const __half *)k_cache_f16, (const __half *)v_cache_f16, (__half *)out_f16, pos0_dev, 1, max_seq, kv_stride, scale, nullptr,
       KvPages{page_table, page_table ? page_shift_of(page_rows) : 0});
   AB200_CHECK_LAUNCH("attention_prefill");
