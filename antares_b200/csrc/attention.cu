@@ -455,10 +455,15 @@ extern "C" int ab200_attention_fused_paged(const void *vqk_f16, const float *inv
   return attention_fused_impl(vqk_f16, inv_freq, pos_dev, k_cache_f16, v_cache_f16, out_f16, H, D, kv_stride, max_seq, scale, page_table, page_rows, stream);
 }
 
-// From how many rows on a prompt goes through the tensor-core kernel.  us, 32 heads, from position 0, the single-query
-// kernel per row against that one: 16 rows 4.2 / 10.9, 32 rows 7.7 / 11.0, 64 rows 14.6 / 10.5, 128 rows 33 / 12.  (The
-// position is a device value, so the rule cannot look at it: behind 500 cached rows the lines cross below 1 row.)
-constexpr int ATT_PREFILL_TC_ROWS = 41;
+// Which prompts go through the tensor-core kernel.  The single-query kernel, once per head and row, takes time by the keys
+// its heads x rows blocks walk, about rows / 2 each and some 30 keys' worth of start; the tensor-core kernel 10.7-12.8 us
+// for anything up to 128 rows.  us, from position 0, single-query / tensor cores:
+//   32 heads  40 rows 8.9 / 11.7, 48 10.6 / 11.7, 56 12.5 / 11.7, 64 14.5 / 10.7, 128 33 / 12.4
+//   16 heads  64 rows 9.5 / 10.7, 96 13.3 / 12.8       8 heads  96 rows 8.7 / 12.9, 128 12.3 / 12.3, 192 19.5 / 12.7
+//    4 heads  128 rows 9.0 / 12.3, 192 13.0 / 12.7     2 heads  192 rows 10.6 / 12.7, 256 13.7 / 14.1, 512 30 / 17.4
+// so the line lies where heads * rows * (rows + 60) is about 190000: 53, 84, 128, 190 and 280 rows.  The position is a device
+// value, so the rule cannot look at it; behind a filled cache the lines cross earlier.
+static bool prefill_on_tensor_cores(int H, int rows) { return (long)H * rows * (rows + 60) >= 190000; }
 
 // Causal attention of `rows` consecutive tokens over a cache that already holds their keys and
 // values: query row r (position *pos0_dev + r) attends cache rows 0 .. *pos0_dev + r.  The batched
@@ -474,7 +479,7 @@ static int attention_prefill_impl(const void *q_f16, const void *k_cache_f16, co
   AB200_REQUIRE(aligned16(q_f16) && aligned16(k_cache_f16) && aligned16(v_cache_f16) && aligned16(out_f16), "attention_prefill: pointers must be 16-byte aligned");
   const size_t smem = ((size_t)max_seq + 16 * ATT_D) * sizeof(float);
   if (smem > 200 * 1024) return fail(AB200_EUNSUPPORTED, "attention_prefill: max_seq=%d exceeds the shared-memory score buffer", max_seq);
-  if (rows >= ATT_PREFILL_TC_ROWS)
+  if (prefill_on_tensor_cores(H, rows))
     return attention_prefill_launch(q_f16, k_cache_f16, v_cache_f16, out_f16, pos0_dev, rows, max_seq, H, kv_stride, scale,
                                     KvPages{page_table, page_table ? page_shift_of(page_rows) : 0}, (cudaStream_t)stream);
   if (smem > 48 * 1024) AB200_CUDA(cudaFuncSetAttribute(attention_decode_kernel<__half, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));

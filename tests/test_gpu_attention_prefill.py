@@ -9,7 +9,7 @@ from antares_b200._lib import call
 from antares_b200 import ops
 
 pytestmark = pytest.mark.gpu
-H, D = 3, 128
+H, D = 48, 128  # with 48 heads the tensor-core kernel takes over at 40 rows
 
 
 def _run(q, k, v, pos0, scale, table=None, page_rows=0, max_seq=None, in_place=False):
@@ -51,8 +51,8 @@ def _close(got, want, v, score=0.0):
     assert bool(((got.double() - want).abs() <= bound).all()), float(((got.double() - want).abs() / bound).max())
 
 
-# edges of the query tile (128) and the key tile (64), both sides of the row rule, one row, prompts behind a filled cache
-@pytest.mark.parametrize("rows,pos0,max_seq", [(1, 0, 64), (8, 3, 64), (16, 0, 16), (40, 0, 64), (41, 0, 64), (41, 22, 63), (41, 900, 941), (63, 0, 64), (64, 1, 65), (65, 0, 80), (127, 0, 200),
+# edges of the query tile (128) and the key tile (64), both sides of the row rule (39 / 40), one row, prompts behind a filled cache
+@pytest.mark.parametrize("rows,pos0,max_seq", [(1, 0, 64), (8, 3, 64), (16, 0, 16), (39, 0, 64), (40, 0, 64), (41, 0, 64), (41, 22, 63), (41, 900, 941), (63, 0, 64), (64, 1, 65), (65, 0, 80), (127, 0, 200),
                                                (128, 0, 128), (129, 0, 129), (200, 300, 512), (451, 0, 451), (30, 1000, 1030)])
 @pytest.mark.parametrize("sharp", [1.0, 24.0])  # 24: scores spread over hundreds, the running maximum moves often
 def test_prefill_attention(rows, pos0, max_seq, sharp):
@@ -110,3 +110,12 @@ def test_result_over_the_queries(rows, value):
     table = torch.arange(80, device="cuda", dtype=torch.int32)
     paged = _run(q, k, v, 0, 0.09, table, 4, 320, in_place=True)
     assert torch.equal(paged.isnan(), want.isnan()) and torch.equal(paged[~want.isnan()], want[~want.isnan()])
+
+
+@pytest.mark.parametrize("heads,rows", [(1, 406), (1, 407), (2, 279), (2, 280), (8, 127), (8, 128), (32, 52), (32, 53)])
+def test_both_sides_of_the_rule(monkeypatch, heads, rows):
+    """Which kernel serves a prompt depends on heads and rows; the result does not."""
+    monkeypatch.setitem(globals(), "H", heads)
+    q, k, v = _inputs(rows, rows + 7, heads)
+    for pos0 in (0, 7):
+        _close(_run(q, k, v, pos0, 0.09), _expected(q, k, v, pos0, 0.09), v)
