@@ -32,7 +32,9 @@
 // pushes its accumulators, 16 rows of x at a time, as fp32 into their owners' shared memory (distributed shared memory,
 // 512 contiguous bytes per warp and store), and after one cluster barrier each CTA adds its own in rank order (bitwise
 // repeatable).  The library owns no scratch for it: a recorded graph holds no pointer that a later call could move.
-// Every mbarrier wait is bounded and reports through the status word (site 210).
+// Every mbarrier wait is bounded and reports through the status word (site 210).  In an early launch the rings fill while the
+// kernel before still runs; no role starts a wait that x has a part in before that kernel is complete, so that the bound is on
+// this kernel alone.
 #include <atomic>
 
 #include <cooperative_groups.h>
@@ -187,6 +189,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
   if (warp == GS_P_WARP) {
     if (gs_elect()) {  // packed words and scales
       for (int u = 0, slot = 0, ph = 1; u < n_units; ++u) {
+        if (u == dp) pdl_wait();  // a slot comes back at the pace of the dequantised ones, those at the pace of the MMAs
         if (u >= dp && !gs_wait(b_pempty + 8 * slot, ph)) {
           good = false;
           break;
@@ -224,6 +227,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
     // Instruction descriptor: D fp32, A/B fp16, B K-major, A K-major or (bit 15) MN-major, N = mt, M = 128
     const uint32_t idesc = (1u << 4) | (TMEM ? 0u : 1u << 15) | ((uint32_t)(mt >> 3) << 17) | (128u >> 4 << 24);
     // One wait and one commit per unit: at some hundred cycles each they, not the MMAs, are what this loop takes.
+    pdl_wait();
     for (int u = 0, xs = 0, ws = 0; u < n_units; ++u) {
       good = __all_sync(0xffffffffu, gs_wait(bar_of(b_full, u), phase_of(u)));
       if (!good) break;
@@ -276,6 +280,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
       // The stage first: once the MMAs of unit u - dw are complete, so is every packed unit up to there, and the packed
       // ring (at least as deep) cannot be two phases behind what this half, which sees every second unit, waits for.  (Nor
       // can the barrier waited on here: the MMAs of unit u - 2 - dw are known to be complete.)
+      if (u == dw || u == dw + 1) pdl_wait();  // the first stage that MMAs have to free
       if (u >= dw) good = __all_sync(0xffffffffu, gs_wait(bar_of(b_used, u - dw), phase_of(u - dw)));
       good = good && __all_sync(0xffffffffu, gs_wait(b_pfull + 8 * ps, pph));
       if (!good) break;

@@ -56,6 +56,10 @@ def test_prompt_gemm_with_swiglu(M, K, F, group):
     # silu's slope is at most 1.1; then one fp16 rounding and a few fp32 steps
     bound = 1.1 * dg * (u.abs() + du) + torch.nn.functional.silu(g).abs() * du + want.abs() * (2 ** -11 + 2 ** -20) + 2 ** -25
     assert bool(((out.double() - want).abs() <= bound).all())
+    # the same as the projections on their own and silu(gate) * up after them: one tiling, one order of sums
+    both, apart = ops.w4a16_gemm(x, q, s), torch.empty_like(out)
+    call("ab200_silu_mul_rows", both.data_ptr(), apart.data_ptr(), M, F, torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(apart, out)
     early = torch.empty_like(out)
     call("ab200_w4a16_gemm_early", x.data_ptr(), q.data_ptr(), s.data_ptr(), early.data_ptr(), M, K, 2 * F, group, 1, torch.cuda.current_stream().cuda_stream)
     assert torch.equal(early, out)
@@ -80,3 +84,26 @@ def test_a_recorded_prompt_gemm_survives_larger_ones():
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, want)
+
+
+@pytest.mark.parametrize("rows,K,N", [(70, 4096, 4096), (300, 4096, 22016), (2000, 4096, 512)])
+def test_early_gemm_behind_a_long_kernel(rows, K, N):
+    """Started at the beginning of a kernel of up to some milliseconds (prompt attention over values that are not finite),
+    whose result it takes: nothing it waits for may run out meanwhile, and it reads the finished result."""
+    H = K // 128
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    qkv = torch.randn(3, rows, H, 128, generator=g, device="cuda").half()
+    qkv[2, 0, 0, 3] = float("inf")
+    pos = torch.zeros(1, device="cuda", dtype=torch.int32)
+    _, q, s = _case(1, K, N, 128, N)
+    stream = torch.cuda.current_stream().cuda_stream
+    ys = []
+    for name, extra in (("ab200_w4a16_gemm_early", 0), ("ab200_w4a16_gemm", 0)):
+        att, y = torch.zeros(rows, K, device="cuda").half(), torch.empty(rows, N, device="cuda").half()
+        torch.cuda.synchronize()
+        call("ab200_attention_prefill", qkv[0].data_ptr(), qkv[1].data_ptr(), qkv[2].data_ptr(), att.data_ptr(), pos.data_ptr(), rows, rows, H, 128, K, 0.09, stream)
+        call(name, att.data_ptr(), q.data_ptr(), s.data_ptr(), y.data_ptr(), rows, K, N, 128, extra, stream)
+        torch.cuda.synchronize()
+        assert ops.kernel_status() == 0 and not att.isfinite().all()
+        ys.append(y)
+    assert torch.equal(ys[0].isnan(), ys[1].isnan()) and torch.equal(ys[0].nan_to_num(), ys[1].nan_to_num())
