@@ -125,14 +125,17 @@ _DT_NAME = {torch.float16: "float16", torch.float32: "float32"}
 _DT_CODE = {"float16": 0, "float32": 1, "int32": 2}
 
 
-def _program(match, kind, order=(), x=0, q=0, stages=(), consts=(), mats=(), cols=()):
+_KIND = {"w4a16": 0, "sigmoid": 1, "softmax": 2, "eltwise": 3, "rowprog": 4}
+
+
+def _program(match, group=0, stages=(), consts=(), mats=(), cols=()):
     """The exported op as the native front end runs it (csrc/fastcall.cpp), or None where it does not; stages:
-    [(kind, postfix program)]; mats / cols: names of the operands in the program's order."""
+    [(kind, postfix program)]; mats / cols: names of the operands in the program's (the entry point's) order."""
     index = {s.name: i for i, s in enumerate(match.inputs)}
     if len(match.inputs) > 8 or any(s.dtype not in _DT_CODE for s in match.inputs):
         return None
     flat = [oa for _, prog in stages for oa in prog]
-    return fast().program(kind, [(_DT_CODE[s.dtype], list(s.dims), [0 if d is None else 1 for d in s.dyn]) for s in match.inputs], list(order), x, q,
+    return fast().program(_KIND[match.kind], [(_DT_CODE[s.dtype], list(s.dims), [0 if d is None else 1 for d in s.dyn]) for s in match.inputs], group,
                           [int(o) for o, _ in flat], [int(a) for _, a in flat], [len(prog) for _, prog in stages], [int(k) for k, _ in stages],
                           [float(c) for c in consts], [index[n] for n in mats], [index[n] for n in cols])
 
@@ -144,13 +147,16 @@ def export(ir, inputs, config=None, name=None):
         pr = match.params
         native = NativeModules(ir, match.inputs, match.output)
         names = [s.name for s in match.inputs]
-        state = []  # the native front end's program, made by the first call
+        # the native front end's program, for calls of any shape: made by the second call, the first one having had the native
+        # boundary accept the text
+        state = []
 
         def fn(*tensors, out=None, extra=None):
-            plain = out is None and len(tensors) == len(names)
-            if plain and state:
+            if state and out is None and len(tensors) == len(names):
+                if state[0] is None:
+                    state[0] = _program(match, pr.get("group", 0), mats=[pr[k] for k in ("x", "qweight", "scales") if k in pr]) or False
                 y = state[0] and fast().run(state[0], *tensors)
-                if y is not None:
+                if y is not None and y is not False:
                     return y
             t, out = _split_call(match, tensors, out)
             ordered = [t[s.name] for s in match.inputs]
@@ -170,9 +176,7 @@ def export(ir, inputs, config=None, name=None):
                 raise ValueError("%s: out must be a contiguous %s tensor of %d elements" % (match.name, x.dtype, torch.Size(shape).numel()))
             native.forward(ordered, out.view(shape) if out.shape != shape else out, _DT_NAME[x.dtype])
             if not state:
-                state.append(_program(match, 0 if match.kind == "w4a16" else 1, native.order, names.index(pr["x"]), names.index(pr["qweight"]) if match.kind == "w4a16" else 0))
-            if plain and state[0]:
-                fast().known(state[0], native.keys[(tuple(tuple(a.shape) for a in ordered), tuple(shape))], *ordered)
+                state.append(None)
             return out
         fn.native = native
     elif match.kind == "eltwise":
@@ -182,7 +186,7 @@ def export(ir, inputs, config=None, name=None):
         def fn(*tensors, out=None, extra=None):
             if out is None and len(tensors) == len(match.inputs):
                 if not state:
-                    state.append(_program(match, 2, stages=[(0, pr["program"])], consts=pr["consts"], mats=pr["inputs"]))
+                    state.append(_program(match, stages=[(0, pr["program"])], consts=pr["consts"], mats=pr["inputs"]))
                 y = state[0] and fast().run(state[0], *tensors)
                 if y is not None:
                     return y
@@ -204,7 +208,7 @@ def export(ir, inputs, config=None, name=None):
         def fn(*tensors, out=None, extra=None):
             if out is None and len(tensors) == len(match.inputs):
                 if not state:
-                    state.append(_program(match, 3, stages=rp["stages"], consts=rp["consts"], mats=rp["mats"], cols=rp["cols"]))
+                    state.append(_program(match, stages=rp["stages"], consts=rp["consts"], mats=rp["mats"], cols=rp["cols"]))
                 y = state[0] and fast().run(state[0], *tensors)
                 if y is not None:
                     return y

@@ -28,7 +28,6 @@ typedef int (*RmsnormVsumFn)(const void *, const void *, const void *, void *, s
 typedef int (*RopeFn)(const void *, const void *, const void *, void *, int, int, int, int, void *);
 typedef int (*RopeAtFn)(const void *, const void *, int, void *, int, int, int, void *);
 typedef int (*AttendAtFn)(const void *, const void *, const void *, void *, int, int, int, long, const void *, int, void *);
-typedef int (*ForwardFn)(int, void *const *, int, void *);
 typedef int (*EltwiseFn)(const void *, const void *, int, const void *, int, const void *, const void *, int, void *, int, size_t, void *);
 typedef int (*RowFn)(const void *, const void *, const void *, const void *, int, const void *, int, const void *, const void *, int, const void *, const void *,
                      int, void *, int, int, int, void *);
@@ -41,7 +40,6 @@ struct Entries {
   RopeFn rope;
   RopeAtFn rope_at;
   AttendAtFn attend_at;
-  ForwardFn forward;
   EltwiseFn eltwise;
   RowFn row;
 } E;
@@ -75,56 +73,66 @@ inline int enter(F f) {  // like ctypes: other threads run during the call
     NOT_HERE;                       \
   }
 
-// w4a16(which, x, qweight, scales): which 0 = by the number of rows, 1 = decode kernels, 2 = tensor-core GEMM
+// x . dequant(q, s); which 0 = by the number of rows, 1 = decode kernels, 2 = tensor-core GEMM; group 0 = what the scales' shape says
+PyObject *project(long which, const Tensor &x, const Tensor &q, const Tensor &s, int64_t group) {
+  const int code = code_of(x);
+  if (code < 0 || s.scalar_type() != x.scalar_type() || q.scalar_type() != at::kInt || q.dim() != 2 || s.dim() != 2 || x.dim() < 1) NOT_HERE;
+  const int64_t K = q.size(0) * 8, N = q.size(1), G = s.size(0);
+  if (K <= 0 || N <= 0 || G <= 0 || K % G || (group && G * group != K) || s.size(1) != N || x.size(-1) != K || x.numel() <= 0) NOT_HERE;
+  const int64_t M = x.numel() / K;
+  if (M > INT32_MAX || K > INT32_MAX || N > INT32_MAX) NOT_HERE;
+  if (which == 0) which = M <= 16 ? 1 : 2;
+  c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
+  shape.back() = N;
+  Tensor out = fresh(shape, x.scalar_type(), x);
+  const GemvFn f = which == 1 ? E.gemv : E.gemm;
+  const void *xp = x.data_ptr(), *qp = q.data_ptr(), *sp = s.data_ptr();
+  void *op = out.data_ptr(), *st = stream();
+  if (enter([&] { return f(xp, qp, sp, op, (int)M, (int)K, (int)N, (int)(K / G), code, st); })) NOT_HERE;
+  return THPVariable_Wrap(std::move(out));
+}
+PyObject *sigmoid_of(const Tensor &x) {
+  const int code = code_of(x);
+  if (code < 0) NOT_HERE;
+  Tensor out = fresh(x.sizes(), x.scalar_type(), x);
+  const void *xp = x.data_ptr();
+  void *op = out.data_ptr(), *st = stream();
+  const size_t count = x.numel();
+  if (enter([&] { return E.sigmoid(xp, op, count, code, st); })) NOT_HERE;
+  return THPVariable_Wrap(std::move(out));
+}
+PyObject *softmax_of(const Tensor &x) {  // over the last axis
+  const int code = code_of(x);
+  if (code < 0 || x.dim() < 1 || x.numel() <= 0) NOT_HERE;
+  const int64_t cols = x.size(-1), rows = x.numel() / cols;
+  if (rows > INT32_MAX || cols > INT32_MAX) NOT_HERE;
+  Tensor out = fresh(x.sizes(), x.scalar_type(), x);
+  const void *xp = x.data_ptr();
+  void *op = out.data_ptr(), *st = stream();
+  if (enter([&] { return E.softmax(xp, op, (int)rows, (int)cols, code, st); })) NOT_HERE;
+  return THPVariable_Wrap(std::move(out));
+}
+
+// w4a16(which, x, qweight, scales), sigmoid(x), softmax(x)
 PyObject *py_w4a16(PyObject *, PyObject *const *a, Py_ssize_t n) {
   GUARDED({
     const Tensor *x, *q, *s;
     if (n != 4 || !(x = plain(a[1])) || !(q = plain(a[2])) || !(s = plain(a[3]))) NOT_HERE;
-    const int code = code_of(*x);
-    if (code < 0 || s->scalar_type() != x->scalar_type() || q->scalar_type() != at::kInt || q->dim() != 2 || s->dim() != 2 || x->dim() < 1) NOT_HERE;
-    const int64_t K = q->size(0) * 8, N = q->size(1), G = s->size(0);
-    if (K <= 0 || N <= 0 || G <= 0 || K % G || s->size(1) != N || x->size(-1) != K || x->numel() <= 0) NOT_HERE;
-    const int64_t M = x->numel() / K;
-    if (M > INT32_MAX || K > INT32_MAX || N > INT32_MAX) NOT_HERE;
-    long which = PyLong_AsLong(a[0]);
-    if (which == 0) which = M <= 16 ? 1 : 2;
-    c10::SmallVector<int64_t, 6> shape(x->sizes().begin(), x->sizes().end());
-    shape.back() = N;
-    Tensor out = fresh(shape, x->scalar_type(), *x);
-    const GemvFn f = which == 1 ? E.gemv : E.gemm;
-    const void *xp = x->data_ptr(), *qp = q->data_ptr(), *sp = s->data_ptr();
-    void *op = out.data_ptr(), *st = stream();
-    if (enter([&] { return f(xp, qp, sp, op, (int)M, (int)K, (int)N, (int)(K / G), code, st); })) NOT_HERE;
-    return THPVariable_Wrap(std::move(out));
+    return project(PyLong_AsLong(a[0]), *x, *q, *s, 0);
   })
 }
-
-// softmax(x) over the last axis, sigmoid(x)
 PyObject *py_sigmoid(PyObject *, PyObject *o) {
   GUARDED({
     const Tensor *x = plain(o);
-    int code;
-    if (!x || (code = code_of(*x)) < 0) NOT_HERE;
-    Tensor out = fresh(x->sizes(), x->scalar_type(), *x);
-    const void *xp = x->data_ptr();
-    void *op = out.data_ptr(), *st = stream();
-    const size_t count = x->numel();
-    if (enter([&] { return E.sigmoid(xp, op, count, code, st); })) NOT_HERE;
-    return THPVariable_Wrap(std::move(out));
+    if (!x) NOT_HERE;
+    return sigmoid_of(*x);
   })
 }
 PyObject *py_softmax(PyObject *, PyObject *o) {
   GUARDED({
     const Tensor *x = plain(o);
-    int code;
-    if (!x || (code = code_of(*x)) < 0 || x->dim() < 1 || x->numel() <= 0) NOT_HERE;
-    const int64_t cols = x->size(-1), rows = x->numel() / cols;
-    if (rows > INT32_MAX || cols > INT32_MAX) NOT_HERE;
-    Tensor out = fresh(x->sizes(), x->scalar_type(), *x);
-    const void *xp = x->data_ptr();
-    void *op = out.data_ptr(), *st = stream();
-    if (enter([&] { return E.softmax(xp, op, (int)rows, (int)cols, code, st); })) NOT_HERE;
-    return THPVariable_Wrap(std::move(out));
+    if (!x) NOT_HERE;
+    return softmax_of(*x);
   })
 }
 
@@ -228,7 +236,7 @@ PyObject *py_attend_at(PyObject *, PyObject *const *a, Py_ssize_t n) {
 }
 
 // ---- exported programs ----------------------------------------------------------------------------------------------
-enum { KIND_W4A16 = 0, KIND_UNARY, KIND_ELTWISE, KIND_ROWS };
+enum { KIND_W4A16 = 0, KIND_SIGMOID, KIND_SOFTMAX, KIND_ELTWISE, KIND_ROWS };
 struct Input {
   at::ScalarType type;
   std::vector<int64_t> bound;
@@ -237,20 +245,13 @@ struct Input {
 struct Program {
   int kind;
   std::vector<Input> inputs;
-  // W4A16 / unary: argument order of the native module, and which input gives the result's shape and columns
-  std::vector<int> order;
-  int x = 0, q = 0;
-  struct Known {
-    std::vector<int64_t> sizes;  // of all inputs, one after the other
-    int key;
-  };
-  std::vector<Known> known;  // the shapes last seen (a few), most recent first
-  // element-wise / row programs: postfix code, operands as indices into the inputs
+  // element-wise / row programs: postfix code, operands as indices into the inputs.  The others: mats holds the operands in
+  // the entry point's order, group the group size that the statements name.
+  int group = 0;
   std::vector<unsigned char> ops, args;
   std::vector<int> lens, kinds, mats, cols;
   std::vector<float> consts;
 };
-constexpr size_t KNOWN_SHAPES = 8;
 
 void drop(PyObject *capsule) { delete static_cast<Program *>(PyCapsule_GetPointer(capsule, "antares_b200.program")); }
 
@@ -263,13 +264,13 @@ bool ints(PyObject *seq, std::vector<T> &v) {
   return !PyErr_Occurred();
 }
 
-// program(kind, [(type, bounds, dyn)], order, x, q, ops, args, lens, kinds, consts, mats, cols)
+// program(kind, [(type, bounds, dyn)], group, ops, args, lens, kinds, consts, mats, cols)
 PyObject *py_program(PyObject *, PyObject *args) {
-  int kind, x, q;
-  PyObject *ins, *order, *ops, *opargs, *lens, *kinds, *consts, *mats, *cols;
-  if (!PyArg_ParseTuple(args, "iOOiiOOOOOOO", &kind, &ins, &order, &x, &q, &ops, &opargs, &lens, &kinds, &consts, &mats, &cols)) return nullptr;
+  int kind, group;
+  PyObject *ins, *ops, *opargs, *lens, *kinds, *consts, *mats, *cols;
+  if (!PyArg_ParseTuple(args, "iOiOOOOOOO", &kind, &ins, &group, &ops, &opargs, &lens, &kinds, &consts, &mats, &cols)) return nullptr;
   auto p = std::make_unique<Program>();
-  p->kind = kind, p->x = x, p->q = q;
+  p->kind = kind, p->group = group;
   PyObject *f = PySequence_Fast(ins, "a sequence of inputs");
   if (!f) return nullptr;
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(f); ++i) {
@@ -285,7 +286,7 @@ PyObject *py_program(PyObject *, PyObject *args) {
   }
   Py_DECREF(f);
   std::vector<int> o, oa;
-  if (!ints(order, p->order) || !ints(ops, o) || !ints(opargs, oa) || !ints(lens, p->lens) || !ints(kinds, p->kinds) || !ints(mats, p->mats) || !ints(cols, p->cols)) return nullptr;
+  if (!ints(ops, o) || !ints(opargs, oa) || !ints(lens, p->lens) || !ints(kinds, p->kinds) || !ints(mats, p->mats) || !ints(cols, p->cols)) return nullptr;
   p->ops.assign(o.begin(), o.end());
   p->args.assign(oa.begin(), oa.end());
   f = PySequence_Fast(consts, "a sequence of constants");
@@ -294,23 +295,6 @@ PyObject *py_program(PyObject *, PyObject *args) {
   Py_DECREF(f);
   if (PyErr_Occurred()) return nullptr;
   return PyCapsule_New(p.release(), "antares_b200.program", drop);
-}
-
-// known(program, key, tensor, ...): remember the native module that serves these shapes
-PyObject *py_known(PyObject *, PyObject *const *a, Py_ssize_t n) {
-  Program *p = n >= 2 ? static_cast<Program *>(PyCapsule_GetPointer(a[0], "antares_b200.program")) : nullptr;
-  if (!p) return nullptr;
-  Program::Known k;
-  k.key = (int)PyLong_AsLong(a[1]);
-  for (Py_ssize_t i = 2; i < n; ++i) {
-    if (!THPVariable_Check(a[i])) NOT_HERE;
-    for (int64_t s : THPVariable_Unpack(a[i]).sizes()) k.sizes.push_back(s);
-  }
-  for (const auto &e : p->known)
-    if (e.sizes == k.sizes) NOT_HERE;
-  p->known.insert(p->known.begin(), std::move(k));
-  if (p->known.size() > KNOWN_SHAPES) p->known.pop_back();
-  NOT_HERE;
 }
 
 constexpr size_t MAX_INPUTS = 8;
@@ -332,31 +316,10 @@ PyObject *py_run(PyObject *, PyObject *const *a, Py_ssize_t n) {
       for (size_t d = 0; d < in.bound.size(); ++d)
         if (t[i]->size(d) > in.bound[d] || (!in.dyn[d] && t[i]->size(d) != in.bound[d])) NOT_HERE;
     }
+    if (p->kind == KIND_W4A16) return project(0, *t[p->mats[0]], *t[p->mats[1]], *t[p->mats[2]], p->group);
+    if (p->kind == KIND_SIGMOID) return sigmoid_of(*t[p->mats[0]]);
+    if (p->kind == KIND_SOFTMAX) return softmax_of(*t[p->mats[0]]);
     void *st = stream();
-    Tensor out;
-    if (p->kind == KIND_W4A16 || p->kind == KIND_UNARY) {
-      int key = -1;
-      for (const auto &k : p->known) {
-        size_t at = 0;
-        bool same = true;
-        for (size_t i = 0; i < count && same; ++i)
-          for (int64_t s : t[i]->sizes()) same = same && at < k.sizes.size() && k.sizes[at++] == s;
-        if (same && at == k.sizes.size()) {
-          key = k.key;
-          break;
-        }
-      }
-      if (key < 0) NOT_HERE;
-      const Tensor &x = *t[p->x];
-      c10::SmallVector<int64_t, 6> shape(x.sizes().begin(), x.sizes().end());
-      if (p->kind == KIND_W4A16) shape.back() = t[p->q]->size(1);
-      out = fresh(shape, x.scalar_type(), x);
-      void *ptr[MAX_INPUTS + 1];
-      for (size_t i = 0; i < count; ++i) ptr[i] = t[p->order[i]]->data_ptr();
-      ptr[count] = out.data_ptr();
-      if (enter([&] { return E.forward(key, ptr, (int)count + 1, st); })) NOT_HERE;
-      return THPVariable_Wrap(std::move(out));
-    }
     bool wide = false;
     const void *mp[MAX_INPUTS], *cp[MAX_INPUTS];
     int md[MAX_INPUTS], cd[MAX_INPUTS];
@@ -374,7 +337,7 @@ PyObject *py_run(PyObject *, PyObject *const *a, Py_ssize_t n) {
       cp[i] = c.data_ptr();
       wide = wide || cd[i] == 1;
     }
-    out = fresh(x.sizes(), wide ? at::kFloat : at::kHalf, x);
+    Tensor out = fresh(x.sizes(), wide ? at::kFloat : at::kHalf, x);
     void *op = out.data_ptr();
     const size_t total = x.numel();
     const int n_consts = (int)p->consts.size();
@@ -403,7 +366,7 @@ PyObject *py_bind(PyObject *, PyObject *d) {
   };
   if (!PyDict_Check(d) || !get("ab200_w4a16_gemv", E.gemv) || !get("ab200_w4a16_gemm", E.gemm) || !get("ab200_sigmoid", E.sigmoid) || !get("ab200_softmax", E.softmax) ||
       !get("ab200_rmsnorm", E.rmsnorm) || !get("ab200_rmsnorm_vsum", E.rmsnorm_vsum) || !get("ab200_rope", E.rope) || !get("ab200_rope_at", E.rope_at) ||
-      !get("ab200_attention_decode_at", E.attend_at) || !get("ab200_forward", E.forward) || !get("ab200_eltwise_vm", E.eltwise) || !get("ab200_rowreduce_vm", E.row))
+      !get("ab200_attention_decode_at", E.attend_at) || !get("ab200_eltwise_vm", E.eltwise) || !get("ab200_rowreduce_vm", E.row))
     return PyErr_Format(PyExc_KeyError, "bind: an entry point is missing");
   Py_RETURN_NONE;
 }
@@ -419,7 +382,6 @@ PyMethodDef methods[] = {{"bind", py_bind, METH_O, nullptr},
                          FAST(rope),
                          FAST(rope_at),
                          FAST(attend_at),
-                         FAST(known),
                          FAST(run),
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_fastcall", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

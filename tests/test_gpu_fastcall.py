@@ -164,3 +164,35 @@ def test_exported_programs(python_only):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(z, y)
+
+
+def test_exported_operators_of_any_shape(monkeypatch):
+    """After the first call, which has the native boundary accept the text, no call of any shape takes the Python route - and what
+    that route refuses for its shapes still is refused."""
+    seen = []
+    forward = autort_api.NativeModules.forward
+    monkeypatch.setattr(autort_api.NativeModules, "forward", lambda self, t, *a: seen.append([tuple(x.shape) for x in t]) or forward(self, t, *a))
+    g = _gen(4)
+    mm = autort.export(ir=autort_api.W4A16_IR_SAMPLE, inputs=["input0=float16[M:40, S:512]", "qweight=int32[L:64, N:512]", "scales=float16[G:8, N:512]"], name="any_mm")
+    sig = autort.export(ir="y[N] = 1 - 1 / (1 + x[N].call(strs.exp))", inputs=["x=float32[N:4096]"], name="any_sig")
+    soft = autort.export(ir="t0[N] >=! x[N, C]; t1[N] +=! (x[N, C] - t0[N]).call(`exp`); y[N, C] = (x[N, C] - t0[N]).call(`exp`) / t1[N]",
+                         inputs=["x=float32[N:64, C:512]"], name="any_soft")
+    for _ in range(2):
+        for i in range(20):
+            K, N, M = 128 * (1 + i % 4), 8 * (3 * i + 1), 1 + 2 * i
+            q, s = _w4(K, N, torch.float16, g)
+            x = torch.randn(M, K, generator=g, device="cuda").half()
+            assert torch.equal(mm(x, q, s), ops.w4a16_matmul(x, q, s))
+            v = torch.randn(100 * i + 1, generator=g, device="cuda")
+            assert torch.equal(sig(v), ops.sigmoid(v))
+            v = torch.randn(i + 1, 8 * (i + 1), generator=g, device="cuda")
+            assert torch.equal(soft(v), ops.softmax(v))
+    assert len(seen) == 3  # one first call each
+    # groups of 64 where the text says 128: the same refusal through either route
+    q, s = _w4(512, 512, torch.float16, g)
+    x, s64 = torch.randn(2, 512, generator=g, device="cuda").half(), s.repeat(2, 1)
+    assert s64.shape == (8, 512)
+    with pytest.raises(Exception, match="W4A16 shapes disagree"):
+        mm(x, q, s64)
+    with pytest.raises(Exception):
+        mm(x[:, :384].contiguous(), q, s)
