@@ -123,17 +123,29 @@ def load():
 _fast = None
 
 
+class _NoFastcall:
+    """Takes no call: the Python code behind every one of them serves it, through the same entry points."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def fast():
-    """The native front end (csrc/fastcall.cpp), its entry points bound.  Raises ImportError if it has not been built."""
+    """The native front end (csrc/fastcall.cpp), its entry points bound.  Where it is missing, or was built for another torch
+    or Python, a warning says so and operators take the Python code behind it: slower per call, the same kernels."""
     global _fast
     if _fast is None:
         L = load()
         try:
-            from . import _fastcall
+            from . import _fastcall, build
+            if _fastcall.built_for() != build.built_for():
+                raise ImportError("built for %s" % _fastcall.built_for())
+            _fastcall.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in SIGNATURES})
+            _fast = _fastcall
         except ImportError as e:
-            raise ImportError("antares_b200/_fastcall.so: %s; run `python -m antares_b200.build`" % e)
-        _fastcall.bind({n: ctypes.cast(getattr(L, n), ctypes.c_void_p).value for n in SIGNATURES})
-        _fast = _fastcall
+            import warnings
+            warnings.warn("antares_b200/_fastcall.so is not used (%s); run `python -m antares_b200.build`" % e)
+            _fast = _NoFastcall()
     return _fast
 
 

@@ -36,23 +36,49 @@ def up_to_date():
     return all(os.path.getmtime(d) <= t for d in deps)
 
 
-def build_fastcall(force=False):
-    if not force and os.path.exists(FAST) and os.path.getmtime(FAST_SRC) <= os.path.getmtime(FAST):
-        return FAST
-    import sysconfig
+def built_for():
+    """What _fastcall.so depends on besides its source: it calls into torch's and Python's binary interfaces."""
     import torch
+    return "torch %s, python %s" % (torch.__version__, sys.version.split()[0])
+
+
+def build_fastcall(force=False):
+    """Needs torch and g++ with Python's headers; the library itself does not, and operators run without it (_lib.fast)."""
+    try:
+        import torch
+    except ImportError as e:
+        sys.stderr.write("antares_b200: _fastcall.so not built (%s)\n" % e)
+        return None
+    import sysconfig
+    note = FAST + ".built_for"
+    if not force and os.path.exists(FAST) and os.path.getmtime(FAST_SRC) <= os.path.getmtime(FAST) and os.path.exists(note):
+        with open(note) as f:
+            if f.read() == built_for():
+                return FAST
     root = os.path.dirname(torch.__file__)
     cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc()))) if os.path.isabs(_nvcc()) else "/usr/local/cuda"
     subprocess.check_call([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-                           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI), "-I" + sysconfig.get_paths()["include"],
+                           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+                           '-DAB200_BUILT_FOR="%s"' % built_for(), "-I" + sysconfig.get_paths()["include"],
                            "-I" + os.path.join(root, "include"), "-I" + os.path.join(root, "include", "torch", "csrc", "api", "include"),
-                           "-I" + os.path.join(cuda, "include"), FAST_SRC, "-o", FAST, "-L" + os.path.join(root, "lib"),
+                           "-I" + os.path.join(cuda, "include"), FAST_SRC, "-o", FAST + ".new", "-L" + os.path.join(root, "lib"),
                            "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python"])
+    os.replace(FAST + ".new", FAST)
+    with open(note, "w") as f:
+        f.write(built_for())
     return FAST
 
 
 def build(force=False, verbose=False):
-    build_fastcall(force)
+    lib = build_library(force, verbose)
+    try:
+        build_fastcall(force)
+    except (OSError, subprocess.CalledProcessError) as e:
+        sys.stderr.write("antares_b200: _fastcall.so not built (%s)\n" % e)
+    return lib
+
+
+def build_library(force=False, verbose=False):
     if not force and up_to_date():
         return LIB
     objs = []

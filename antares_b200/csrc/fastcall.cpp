@@ -371,8 +371,12 @@ PyObject *py_bind(PyObject *, PyObject *d) {
   Py_RETURN_NONE;
 }
 
+// what this file was compiled against; another torch or Python must not use it
+PyObject *py_built_for(PyObject *, PyObject *) { return PyUnicode_FromString(AB200_BUILT_FOR); }
+
 #define FAST(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {{"bind", py_bind, METH_O, nullptr},
+                         {"built_for", py_built_for, METH_NOARGS, nullptr},
                          {"program", py_program, METH_VARARGS, nullptr},
                          {"sigmoid", py_sigmoid, METH_O, nullptr},
                          {"softmax", py_softmax, METH_O, nullptr},
