@@ -76,14 +76,11 @@ def _split_call(match, tensors, out):
     return by_name, out
 
 
-def _settle(given, used):
-    """Called before a W4A16 launch with the weights a caller gave and those the launch reads.  The fp16 decode kernels bring
-    weights and scales in before they wait for the kernel ahead of them, so that one must not be the copy that made them
-    contiguous: a fill in between does not start before the copy is complete and visible."""
-    for a, b in zip(given, used):
-        if a is not b and b.is_cuda:
-            torch.zeros(1, device=b.device)
-            return
+def _settle(device):
+    """Called before a W4A16 launch whose weights or scales had to be made contiguous.  The fp16 decode kernels bring both in before
+    they wait for the kernel ahead of them, so that one must not be the copy: a fill in between does not start before the copy
+    is complete and visible."""
+    torch.zeros(1, device=device)
 
 
 class NativeModules:
@@ -147,6 +144,7 @@ def export(ir, inputs, config=None, name=None):
         pr = match.params
         native = NativeModules(ir, match.inputs, match.output)
         names = [s.name for s in match.inputs]
+        qi, si = (names.index(pr[k]) for k in ("qweight", "scales")) if match.kind == "w4a16" else (0, 0)
         # the native front end's program, for calls of any shape: made by the second call, the first one having had the native
         # boundary accept the text
         state = []
@@ -167,7 +165,8 @@ def export(ir, inputs, config=None, name=None):
             if match.kind == "w4a16":
                 qw = t[pr["qweight"]]
                 shape = tuple(x.shape[:-1]) + (qw.shape[1],)
-                _settle(*zip(*((a, b) for n, a, b in zip(names, tensors, ordered) if n != pr["x"])))
+                if ordered[qi] is not tensors[qi] or ordered[si] is not tensors[si]:
+                    _settle(x.device)
             else:
                 shape = tuple(x.shape)
             if out is None:

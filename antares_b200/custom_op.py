@@ -44,7 +44,8 @@ class CustomOp(torch.nn.Module):
         if self.match.kind in ("w4a16", "sigmoid", "softmax"):
             # the named family goes through the native plugin boundary (ab200_inject / ab200_forward), as the
             # reference's forward() goes through custom_lib.inject / custom_lib.forward (custom_op.py:117-148)
-            from .autort_api import NativeModules
+            from .autort_api import NativeModules, _settle
+            self.settle = _settle
             self.native = NativeModules(self.ir, self.match.inputs, self.match.output)
         return self
 
@@ -60,9 +61,8 @@ class CustomOp(torch.nn.Module):
             shape = tuple(x.shape[:-1]) + (t[pr["qweight"]].shape[1],) if self.match.kind == "w4a16" else tuple(x.shape)
             out = torch.empty(shape, dtype=x.dtype, device=x.device)
             dt = {torch.float16: "float16", torch.float32: "float32"}[x.dtype]
-            if self.match.kind == "w4a16":
-                from .autort_api import _settle
-                _settle(*zip(*((a, t[k]) for k, a in zip(self.input_names, inputs) if k != pr["x"])))
+            if self.match.kind == "w4a16" and any(t[k] is not a for k, a in zip(self.input_names, inputs) if k != pr["x"]):
+                self.settle(x.device)
             return self.native.forward([t[s.name] for s in self.match.inputs], out, dt)
         if self.match.kind == "eltwise":
             ins = [t[n] for n in pr["inputs"]]
