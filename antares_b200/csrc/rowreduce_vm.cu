@@ -9,7 +9,7 @@
 // elements of a thread at a time; a reduction stage folds the values of a row with + / max / min (warp shuffles,
 // one shared-memory hop, fixed order, so results are bitwise repeatable), the final stage writes the output.  The
 // row stays in L1/L2 between stages, so HBM sees each input once.  Instruction issue is what bounds it: layernorm with
-// weight and bias over 2048 x 4096 fp16 takes 53 us (300 before, one element per decode) for 5 us of traffic.  The block is as wide as the row needs (32 to 256
+// weight and bias over 2048 x 4096 fp16 takes 46 us (296 with one element per decode) for 5 us of traffic.  The block is as wide as the row needs (32 to 256
 // threads), so short rows do not leave warps idle.
 #include <math_constants.h>
 
@@ -22,29 +22,29 @@ constexpr int RV_MAX_THREADS = 256;
 
 enum { RV_MAP = 0, RV_SUM = 1, RV_RMAX = 2, RV_RMIN = 3 };
 
+// All stages' instructions lie one after the other, a stage's temporaries (what it computes once per row) before its own:
+// temporary i of stage s is code[begin[s][i]] .. code[begin[s][i + 1]), the stage itself the piece after the last of them.
+constexpr int RV_MAX_CODE = RV_MAX_STAGES * 2 * VM_MAX_OPS;
 struct RowProgram {
+  int rows, cols;
+  unsigned char n_stages, vec_ok, out_f16, reduce[RV_MAX_STAGES], n_temps[RV_MAX_STAGES];
+  unsigned char mat_f16[RV_MAX_MAT], col_f16[RV_MAX_COL];
+  unsigned short begin[RV_MAX_STAGES][VM_MAX_TEMPS + 2];
   const void *mat[RV_MAX_MAT];  // [rows, cols]
   const void *col[RV_MAX_COL];  // [cols]
   void *out;                    // [rows, cols]
   float cst[VM_MAX_CONSTS];
-  unsigned code[RV_MAX_STAGES][VM_MAX_OPS];
-  VmTemps temps[RV_MAX_STAGES];  // what a stage computes once per row
-  unsigned char n_code[RV_MAX_STAGES], reduce[RV_MAX_STAGES];
-  unsigned char mat_f16[RV_MAX_MAT], col_f16[RV_MAX_COL];
-  int n_stages, out_f16, rows, cols, vec_ok;
+  VmCode code[RV_MAX_CODE];
 };
 
+// The instructions are read from the parameters: copied to shared memory first they were slower in every size (layernorm of
+// 2048 x 4096 51.7 against 48.4 us), the copy being a start-up of a microsecond or more per block (4096 x 256: 22 against
+// 10.8 us; with half-word instructions packed end to end 45.7 and 10.1).
 __global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const __grid_constant__ RowProgram p) {
   extern __shared__ float4 vm_stack[];
   // [row parity]: a warp that is a row ahead writes the other half (every row with a reduction has a barrier)
   __shared__ float part[2][RV_MAX_STAGES][RV_MAX_THREADS / 32];
   __shared__ float temp[RV_MAX_STAGES][VM_MAX_TEMPS];
-  __shared__ unsigned code[RV_MAX_STAGES][VM_MAX_OPS], pre[RV_MAX_STAGES][VM_MAX_OPS];
-  for (int i = threadIdx.x; i < RV_MAX_STAGES * VM_MAX_OPS; i += blockDim.x) {
-    (&code[0][0])[i] = p.code[i / VM_MAX_OPS][i % VM_MAX_OPS];
-    (&pre[0][0])[i] = p.temps[i / VM_MAX_OPS].code[i % VM_MAX_OPS];
-  }
-  __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned threads = blockDim.x, step = p.vec_ok ? 1 : threads;
   const int per_pass = (int)threads * VM_E;
@@ -53,18 +53,18 @@ __global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const _
     const size_t base = (size_t)row * p.cols;
     float r0 = 0.f, r1 = 0.f, r2 = 0.f;  // results of the reduction stages
     for (int s = 0; s < p.n_stages; ++s) {
-      const int kind = p.reduce[s];
+      const int kind = p.reduce[s], n_temps = p.n_temps[s];
+      const unsigned short *begin = p.begin[s];
       auto scalar = [&](unsigned k, unsigned arg) {
         return k == VM_K_CONST ? p.cst[arg] : k == VM_K_COLLEN ? (float)p.cols : k == VM_K_TEMP ? temp[s][arg] : arg == 0 ? r0 : arg == 1 ? r1 : r2;
       };
-      if (p.temps[s].n) {  // one warp's work; every warp on its own would spend a third of the row's instructions on it
+      if (n_temps) {  // one warp's work; every warp on its own would spend a third of the row's instructions on it
         if (warp == 0) {
 #pragma unroll 1
-          for (int i = 0; i < p.temps[s].n; ++i) {
+          for (int i = 0; i < n_temps; ++i) {
             float v[1];
             const float none[1] = {0.f};
-            vm_run<1>(pre[s] + p.temps[s].start[i], p.temps[s].start[i + 1] - p.temps[s].start[i], vm_stack + threadIdx.x, threads, v, none, scalar,
-                      [](unsigned, unsigned, float(&)[1]) {});
+            vm_run<1>(p.code + begin[i], begin[i + 1] - begin[i], vm_stack + threadIdx.x, threads, v, none, scalar, [](unsigned, unsigned, float(&)[1]) {});
             if (lane == 0) temp[s][i] = v[0];
           }
         }
@@ -78,7 +78,7 @@ __global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const _
         const bool vec = p.vec_ok && count == VM_E;
         float first[VM_E], t[VM_E];
         vm_load(p.mat[0], p.mat_f16[0], base + c, step, count, vec, first);
-        vm_run<VM_E>(code[s], p.n_code[s], vm_stack + threadIdx.x, threads, t, first, scalar, [&](unsigned k, unsigned arg, float(&b)[VM_E]) {
+        vm_run<VM_E>(p.code + begin[n_temps], begin[n_temps + 1] - begin[n_temps], vm_stack + threadIdx.x, threads, t, first, scalar, [&](unsigned k, unsigned arg, float(&b)[VM_E]) {
           if (k == VM_K_COL) vm_load(p.col[arg], p.col_f16[arg], c, step, count, vec, b);
           else vm_load(p.mat[arg], p.mat_f16[arg], base + c, step, count, vec, b);
         });
@@ -145,7 +145,7 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
   }
   for (int i = 0; i < n_consts; ++i) p.cst[i] = consts_host[i];
   // validate every stage on the host: operand indices, stack discipline, stage order
-  int off = 0, stack = 0;
+  int off = 0, stack = 0, total = 0;
   for (int s = 0; s < n_stages; ++s) {
     const int len = stage_len_host[s], kind = stage_reduce_host[s];
     AB200_REQUIRE(len >= 1 && len <= VM_MAX_OPS, "rowreduce_vm: stage %d has %d operations (1..%d)", s, len, VM_MAX_OPS);
@@ -171,7 +171,14 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
     }
     AB200_REQUIRE(depth == 1, "rowreduce_vm: stage %d leaves %d values on the stack", s, depth);
     int depth_used = 0;
-    p.n_code[s] = (unsigned char)vm_translate(ops_host + off, args_host + off, len, p.code[s], &depth_used, &p.temps[s]);
+    VmTemps temps;
+    VmCode code[VM_MAX_OPS];
+    const int n = vm_translate(ops_host + off, args_host + off, len, code, &depth_used, &temps);
+    p.n_temps[s] = temps.n;
+    for (int i = 0; i <= temps.n; ++i) p.begin[s][i] = (unsigned short)(total + temps.start[i]);
+    for (int i = 0; i < temps.start[temps.n]; ++i) p.code[total++] = temps.code[i];
+    for (int i = 0; i < n; ++i) p.code[total++] = code[i];
+    p.begin[s][temps.n + 1] = (unsigned short)total;
     if (depth_used > stack) stack = depth_used;
     p.reduce[s] = (unsigned char)kind;
     off += len;
@@ -188,7 +195,7 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
   while (threads < RV_MAX_THREADS && threads * VM_E < cols) threads *= 2;
   const int cap = sm_count() * (2048 / threads);
   const size_t smem = (size_t)stack * threads * VM_E * sizeof(float);
-  // the limit that needs no opting in, 48 KiB, is on this and the static arrays (under 2 KiB) together
+  // the limit that needs no opting in, 48 KiB, is on this and the static arrays together
   if (smem > 46 * 1024) AB200_CUDA(cudaFuncSetAttribute(rowreduce_vm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   rowreduce_vm_kernel<<<rows < cap ? rows : cap, threads, smem, (cudaStream_t)stream>>>(p);
   AB200_CHECK_LAUNCH("rowreduce_vm");

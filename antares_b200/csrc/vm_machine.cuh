@@ -27,22 +27,25 @@ enum VmOp : unsigned {
 __host__ __device__ constexpr bool vm_is_leaf(unsigned op) { return op <= VM_CONST || (op >= VM_ROW && op <= VM_COLLEN); }
 __host__ __device__ constexpr bool vm_is_binary(unsigned op) { return (op >= VM_ADD && op <= VM_DIV) || (op >= VM_MAX && op <= VM_POW); }
 
-// an instruction: operation | operand kind << 8 | operand index << 12 | push << 20
+// an instruction: operation | operand kind << 5 | operand index << 8 | push << 12.  Half words: a small launch waits for every
+// line of its parameters that it touches.
+typedef unsigned short VmCode;
 enum { VM_K_NONE = 0, VM_K_POP, VM_K_CONST, VM_K_IN, VM_K_ROW, VM_K_COL, VM_K_COLLEN, VM_K_TEMP };
-constexpr unsigned VM_PUSH = 1u << 20;
+constexpr unsigned VM_PUSH = 1u << 12;
 
 constexpr int VM_MAX_TEMPS = 4;
+static_assert(VM_LOAD < 32 && VM_K_TEMP < 8 && VM_MAX_CONSTS <= 16 && VM_MAX_TEMPS <= 16, "an instruction's fields");
 
 // Programs that run once per row: temp i is the value of pre[start[i]] .. pre[start[i + 1]).
 struct VmTemps {
-  unsigned code[VM_MAX_OPS];
+  VmCode code[VM_MAX_OPS];
   unsigned char start[VM_MAX_TEMPS + 1];
   unsigned char n;
 };
 
 // Host: a valid postfix program -> instructions; returns how many, and the deepest stack in *depth.  temps: where the
 // subexpressions without vector operands go (nullptr: they stay).
-inline int vm_translate(const unsigned char *op, const unsigned char *arg, int n, unsigned *code, int *depth, VmTemps *temps = nullptr) {
+inline int vm_translate(const unsigned char *op, const unsigned char *arg, int n, VmCode *code, int *depth, VmTemps *temps = nullptr) {
   int start[VM_MAX_OPS], temp[VM_MAX_OPS], top_of[VM_MAX_OPS], sp = 0;  // start[k]: first operation of the subexpression that k closes
   bool scalar[VM_MAX_OPS];
   for (int k = 0; k < n; ++k) {
@@ -64,19 +67,19 @@ inline int vm_translate(const unsigned char *op, const unsigned char *arg, int n
   struct Emit {
     const unsigned char *op, *arg;
     const int *start, *temp;
-    unsigned *code;
+    VmCode *code;
     int n, live, deepest;
     bool simple(int k) const { return vm_is_leaf(op[k]) || temp[k] >= 0; }
     unsigned operand(int k) const {
-      if (temp[k] >= 0) return VM_K_TEMP << 8 | (unsigned)temp[k] << 12;
+      if (temp[k] >= 0) return VM_K_TEMP << 5 | (unsigned)temp[k] << 8;
       const unsigned kind = op[k] == VM_IN ? VM_K_IN : op[k] == VM_CONST ? VM_K_CONST : op[k] == VM_ROW ? VM_K_ROW : op[k] == VM_COL ? VM_K_COL : VM_K_COLLEN;
-      return kind << 8 | (unsigned)arg[k] << 12;
+      return kind << 5 | (arg[k] & 15u) << 8;
     }
     static unsigned reversed(unsigned o) { return o == VM_SUB ? VM_RSUB : o == VM_DIV ? VM_RDIV : o == VM_POW ? VM_RPOW : o; }
     void eval(int k, bool push) {  // push: the value in `top` is needed later, save it before the first load
       if (simple(k)) {
         if (push && ++live > deepest) deepest = live;
-        code[n++] = (unsigned)VM_LOAD | operand(k) | (push ? VM_PUSH : 0u);
+        code[n++] = (VmCode)((unsigned)VM_LOAD | operand(k) | (push ? VM_PUSH : 0u));
       } else if (!vm_is_binary(op[k])) {
         eval(k - 1, push);
         code[n++] = op[k];
@@ -84,15 +87,15 @@ inline int vm_translate(const unsigned char *op, const unsigned char *arg, int n
         const int r = k - 1, l = start[r] - 1;
         if (simple(r)) {
           eval(l, push);
-          code[n++] = op[k] | operand(r);
+          code[n++] = (VmCode)(op[k] | operand(r));
         } else if (simple(l)) {
           eval(r, push);
-          code[n++] = reversed(op[k]) | operand(l);
+          code[n++] = (VmCode)(reversed(op[k]) | operand(l));
         } else {
           eval(l, push);
           eval(r, true);
           --live;
-          code[n++] = reversed(op[k]) | (unsigned)VM_K_POP << 8;
+          code[n++] = (VmCode)(reversed(op[k]) | (unsigned)VM_K_POP << 5);
         }
       }
     }
@@ -188,7 +191,7 @@ __device__ __forceinline__ void vm_store(void *p, bool f16, size_t i, unsigned s
 // read ahead, and the commonest operations are tested before the jump table, with a scalar or the first input without a
 // copy of the operand.
 template <int EN, class Scalar, class Vector>
-__device__ __forceinline__ void vm_run(const unsigned *code, int n, float4 *stack, unsigned threads, float (&t)[EN], const float (&first)[EN], Scalar scalar,
+__device__ __forceinline__ void vm_run(const VmCode *code, int n, float4 *stack, unsigned threads, float (&t)[EN], const float (&first)[EN], Scalar scalar,
                                        Vector vector) {
   constexpr int QUADS = (EN + 3) / 4;
 #define VM_EACH(expr)                             \
@@ -219,7 +222,7 @@ __device__ __forceinline__ void vm_run(const unsigned *code, int n, float4 *stac
   }
   unsigned ahead = code[0];
   for (int k = 0; k < n; ++k) {
-    const unsigned w = ahead, o = w & 255u, kind = (w >> 8) & 15u, arg = (w >> 12) & 255u;
+    const unsigned w = ahead, o = w & 31u, kind = (w >> 5) & 7u, arg = (w >> 8) & 15u;
     if (k + 1 < n) ahead = code[k + 1];
     float b[EN];
     if (w & VM_PUSH) {
