@@ -80,6 +80,9 @@ __device__ __forceinline__ uint32_t gs_smem_u32(const void *p) { return (uint32_
 __device__ __forceinline__ uint64_t gs_desc(uint32_t addr, uint32_t lead) {
   return (uint64_t)((addr >> 4) & 0x3FFF) | (uint64_t)((lead >> 4) & 0x3FFF) << 16 | (uint64_t)(1024 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)2 << 61;
 }
+// X: x has a part in what is waited for.  In an early launch the polls, which are counted, then begin when the kernel before is
+// complete.
+template <bool X>
 __device__ __forceinline__ bool gs_wait(uint32_t bar, unsigned parity) {
   {  // non-blocking probe first: cheaper than try_wait when the phase completed long ago
     uint32_t done;
@@ -90,6 +93,7 @@ __device__ __forceinline__ bool gs_wait(uint32_t bar, unsigned parity) {
         : "memory");
     if (done) return true;
   }
+  if (X) pdl_wait();
   for (unsigned i = 0; i < GS_WAIT_POLLS; ++i) {
     uint32_t done;
     asm volatile(
@@ -189,8 +193,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
   if (warp == GS_P_WARP) {
     if (gs_elect()) {  // packed words and scales
       for (int u = 0, slot = 0, ph = 1; u < n_units; ++u) {
-        if (u == dp) pdl_wait();  // a slot comes back at the pace of the dequantised ones, those at the pace of the MMAs
-        if (u >= dp && !gs_wait(b_pempty + 8 * slot, ph)) {
+        if (u >= dp && !gs_wait<true>(b_pempty + 8 * slot, ph)) {
           good = false;
           break;
         }
@@ -210,7 +213,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
     if (gs_elect()) {  // x tiles
       pdl_wait();      // x comes from the kernel before this one; weights and scales may be on their way already (p.early)
       for (int u = 0, slot = 0; u < n_units; ++u) {
-        if (u >= dx && !gs_wait(bar_of(b_used, u - dx), phase_of(u - dx))) {
+        if (u >= dx && !gs_wait<true>(bar_of(b_used, u - dx), phase_of(u - dx))) {
           good = false;
           break;
         }
@@ -227,9 +230,8 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
     // Instruction descriptor: D fp32, A/B fp16, B K-major, A K-major or (bit 15) MN-major, N = mt, M = 128
     const uint32_t idesc = (1u << 4) | (TMEM ? 0u : 1u << 15) | ((uint32_t)(mt >> 3) << 17) | (128u >> 4 << 24);
     // One wait and one commit per unit: at some hundred cycles each they, not the MMAs, are what this loop takes.
-    pdl_wait();
     for (int u = 0, xs = 0, ws = 0; u < n_units; ++u) {
-      good = __all_sync(0xffffffffu, gs_wait(bar_of(b_full, u), phase_of(u)));
+      good = __all_sync(0xffffffffu, gs_wait<true>(bar_of(b_full, u), phase_of(u)));
       if (!good) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint64_t b0 = gs_desc(s_x + xs * xb, 16);
@@ -280,9 +282,8 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
       // The stage first: once the MMAs of unit u - dw are complete, so is every packed unit up to there, and the packed
       // ring (at least as deep) cannot be two phases behind what this half, which sees every second unit, waits for.  (Nor
       // can the barrier waited on here: the MMAs of unit u - 2 - dw are known to be complete.)
-      if (u == dw || u == dw + 1) pdl_wait();  // the first stage that MMAs have to free
-      if (u >= dw) good = __all_sync(0xffffffffu, gs_wait(bar_of(b_used, u - dw), phase_of(u - dw)));
-      good = good && __all_sync(0xffffffffu, gs_wait(b_pfull + 8 * ps, pph));
+      if (u >= dw) good = __all_sync(0xffffffffu, gs_wait<true>(bar_of(b_used, u - dw), phase_of(u - dw)));
+      good = good && __all_sync(0xffffffffu, gs_wait<false>(b_pfull + 8 * ps, pph));
       if (!good) break;
       uint32_t w[8];
       uint4 sv = make_uint4(0, 0, 0, 0);
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(GS_THREADS, 1) w4a16_gemm_tcgen05_kernel(const
   }
   pdl_wait();  // (long satisfied) out may still have been in use
   // ---- all MMAs of this CTA are done, its shared memory is idle -----------------------------------------------------
-  if (!gs_wait(b_done, 0)) fail_s = 1;
+  if (!gs_wait<true>(b_done, 0)) fail_s = 1;
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   __syncthreads();
   const bool failed = fail_s != 0;
