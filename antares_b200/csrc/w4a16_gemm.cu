@@ -475,7 +475,10 @@ static int gemm_launch(const void *x, const int32_t *qweight, const void *scales
   // Row tiles: at least M / 256; more and narrower ones when that fills the last round of CTAs better.  K split, when the
   // tiles leave SMs idle: as many parts as keep every tile's cluster resident at once (a cluster lies within one GPC, so
   // this is not SMs / parts), each of at least 4 units.  A unit costs about what was measured for the two
-  // forms; a tile costs its start and epilogue, a split the exchange of its rows.
+  // forms; a tile costs its start and epilogue, a split the exchange of its rows.  Unsplit, K = 4096, a round of all SMs takes
+  // 33 / 35 / 37 us at 112 / 128 / 160 rows, 44 / 45 at 176 / 192 (tensor memory then has two stages of weights in place of
+  // three) and 47.5 / 50 / 51.5 with the weights in shared memory at 208 / 240 / 256.  2048 rows of N 12288 / 22016 take 161 / 298 us
+  // so (9 and 8 tiles), 183 / 343 with the former's costs taken for both (12 tiles of 176), 187 / 331 the kernel before this one.
   const int tiles_n = silu ? (N / 2 + GS_BN / 2 - 1) / (GS_BN / 2) : (N + GS_BN - 1) / GS_BN, units = K / GS_BK, sms = sm_count();
   auto rows_of = [&](int tiles_m) { return ((M + tiles_m - 1) / tiles_m + 15) / 16 * 16; };
   auto parts_of = [&](long tiles) {
@@ -485,7 +488,8 @@ static int gemm_launch(const void *x, const int32_t *qweight, const void *scales
   };
   auto cost = [&](int tiles_m) {
     const long tiles = (long)tiles_n * tiles_m, rounds = (tiles + sms - 1) / sms;
-    const int rows = rows_of(tiles_m), unit = rows <= GS_TMEM_MT ? 650 + 2 * rows : 700 + 3 * rows, parts = parts_of(tiles);
+    const int rows = rows_of(tiles_m), parts = parts_of(tiles);
+    const int unit = rows > GS_TMEM_MT ? (parts == 1 ? 770 + 5 * rows / 2 : 700 + 3 * rows) : 650 + 2 * rows + (parts == 1 && rows > 160 ? 170 : 0);
     return rounds * ((long)((units + parts - 1) / parts) * unit + GS_TILE_CYCLES + (parts > 1 ? GS_SPLIT_CYCLES + rows * GS_SPLIT_ROW_CYCLES : 0));
   };
   const int least = (M + GS_MAX_MT - 1) / GS_MAX_MT;
