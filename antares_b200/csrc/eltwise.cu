@@ -94,7 +94,7 @@ __global__ void sigmoid_kernel(const T *__restrict__ x, T *__restrict__ out, siz
 // so the global-load latency of one row hides behind the reduction and the stores of the one before.
 // The norm weights of a thread's columns are loaded once.  VEC = 8-element vectors per thread.
 // ADD: the row is the residual stream, x += y (y fp16) is stored back on the way: the prompt pass's residual update
-// and the norm that follows it in one pass (80 + 48 bytes per 8 elements moved apart, 80 together).
+// and the norm that follows it in one pass (80 + 48 bytes per 8 elements moved apart, 96 together).
 template <typename T, int VEC, bool ADD = false>
 __global__ void __launch_bounds__(ROW_THREADS) rmsnorm_rows_kernel(std::conditional_t<ADD, T, const T> *__restrict__ x, const __half *__restrict__ w,
                                                                   __half *__restrict__ out, int rows, int cols, float eps, const __half *__restrict__ y = nullptr) {

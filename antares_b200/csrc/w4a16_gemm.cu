@@ -24,8 +24,8 @@
 // What bounds them: with weights and x both in shared memory a unit moves 3 mt + 700 cycles' worth of it (128 bytes a
 // cycle) for 4 mt cycles of MMA; with the weights in tensor memory it is the eight MMAs of a unit, which take 85 to 100
 // cycles each however small mt is, 650 + 2 mt a unit in all.  Measured, us, K 4096 N 12288 / 22016: 128 rows 22 / 33, and
-// 48 / 37 with the weights in shared memory; 2048 rows, both forms in play, 163-167 / 290-298.  The kernel before this one
-// (x as the M operand padded to 128, K split through global scratch): 43 / 43 and 170 / 290.
+// 48 / 37 with the weights in shared memory; 2048 rows 161 / 298.  The kernel before this one (x as the M operand padded to
+// 128, K split through global scratch): 43 / 43 and, in the same runs, 187 / 331.
 // Roles: 2 x 8 dequantising warps (units alternate between the two halves), one thread each for the x copies and the
 // packed copies, one warp for the MMAs; they meet through mbarriers.
 // K split: the parts of a tile are the CTAs of one thread-block cluster (at most 8).  After the last MMA every CTA

@@ -322,7 +322,7 @@ class LlamaInt4Decoder:
             self._prefill_pass(T, self._prefill_buffers(T))
         elif cached is None:
             # first prompt of this length: run the pass eagerly, then record it as a CUDA graph over the same
-            # buffers (352 launches at 32 layers: replayed, the pass is bound by the GPU, not by the host)
+            # buffers (eight launches a layer: replayed, the pass is bound by the GPU, not by the host)
             bufs = self._prefill_buffers(T)
             self._prefill_pass(T, bufs)
             side = torch.cuda.Stream(device=self.dev)
