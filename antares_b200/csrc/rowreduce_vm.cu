@@ -6,7 +6,7 @@
 // kernel runs all stages of a row back to back: every stage's expression is a small postfix program
 // (the same operation set as the element-wise interpreter, plus "row value of an earlier stage",
 // "column vector" and "number of columns"), run by the accumulator machine of vm_machine.cuh in fp32, eight
-// elements of a thread at a time; a reduction stage folds the values of a row with + / max / min (warp shuffles,
+// elements of a thread at a time (one in small launches); a reduction stage folds the values of a row with + / max / min (warp shuffles,
 // one shared-memory hop, fixed order, so results are bitwise repeatable), the final stage writes the output.  The
 // row stays in L1/L2 between stages, so HBM sees each input once.  Instruction issue is what bounds it: layernorm with
 // weight and bias over 2048 x 4096 fp16 takes 46 us (296 with one element per decode) for 5 us of traffic.  The block is as wide as the row needs (32 to 256
@@ -40,6 +40,7 @@ struct RowProgram {
 // The instructions are read from the parameters: copied to shared memory first they were slower in every size (layernorm of
 // 2048 x 4096 51.7 against 48.4 us), the copy being a start-up of a microsecond or more per block (4096 x 256: 22 against
 // 10.8 us; with half-word instructions packed end to end 45.7 and 10.1).
+template <int E>
 __global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const __grid_constant__ RowProgram p) {
   extern __shared__ float4 vm_stack[];
   // [row parity]: a warp that is a row ahead writes the other half (every row with a reduction has a barrier)
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const _
   __shared__ float temp[RV_MAX_STAGES][VM_MAX_TEMPS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const unsigned threads = blockDim.x, step = p.vec_ok ? 1 : threads;
-  const int per_pass = (int)threads * VM_E;
+  const int per_pass = (int)threads * E;
   int parity = 0;
   for (int row = blockIdx.x; row < p.rows; row += gridDim.x, parity ^= 1) {
     const size_t base = (size_t)row * p.cols;
@@ -72,13 +73,13 @@ __global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const _
       }
       float acc = kind == RV_RMAX ? -CUDART_INF_F : kind == RV_RMIN ? CUDART_INF_F : 0.f;
       for (int c0 = 0; c0 < p.cols; c0 += per_pass) {
-        const int c = c0 + (int)threadIdx.x * (p.vec_ok ? VM_E : 1);
+        const int c = c0 + (int)threadIdx.x * (p.vec_ok ? E : 1);
         const int left = c < p.cols ? (p.cols - c + (int)step - 1) / (int)step : 0;
-        const int count = left < VM_E ? left : VM_E;
-        const bool vec = p.vec_ok && count == VM_E;
-        float first[VM_E], t[VM_E];
+        const int count = left < E ? left : E;
+        const bool vec = p.vec_ok && count == E;
+        float first[E], t[E];
         vm_load(p.mat[0], p.mat_f16[0], base + c, step, count, vec, first);
-        vm_run<VM_E>(p.code + begin[n_temps], begin[n_temps + 1] - begin[n_temps], vm_stack + threadIdx.x, threads, t, first, scalar, [&](unsigned k, unsigned arg, float(&b)[VM_E]) {
+        vm_run<E>(p.code + begin[n_temps], begin[n_temps + 1] - begin[n_temps], vm_stack + threadIdx.x, threads, t, first, scalar, [&](unsigned k, unsigned arg, float(&b)[E]) {
           if (k == VM_K_COL) vm_load(p.col[arg], p.col_f16[arg], c, step, count, vec, b);
           else vm_load(p.mat[arg], p.mat_f16[arg], base + c, step, count, vec, b);
         });
@@ -86,13 +87,13 @@ __global__ void __launch_bounds__(RV_MAX_THREADS, 4) rowreduce_vm_kernel(const _
           vm_store(p.out, p.out_f16, base + c, step, count, vec, t);
         } else if (kind == RV_SUM) {
 #pragma unroll
-          for (int j = 0; j < VM_E; ++j) acc += j < count ? t[j] : 0.f;
+          for (int j = 0; j < E; ++j) acc += j < count ? t[j] : 0.f;
         } else if (kind == RV_RMAX) {
 #pragma unroll
-          for (int j = 0; j < VM_E; ++j) acc = j < count ? fmaxf(acc, t[j]) : acc;
+          for (int j = 0; j < E; ++j) acc = j < count ? fmaxf(acc, t[j]) : acc;
         } else {
 #pragma unroll
-          for (int j = 0; j < VM_E; ++j) acc = j < count ? fminf(acc, t[j]) : acc;
+          for (int j = 0; j < E; ++j) acc = j < count ? fminf(acc, t[j]) : acc;
         }
       }
       if (kind != RV_MAP) {
@@ -191,13 +192,21 @@ extern "C" int ab200_rowreduce_vm(const unsigned char *ops_host, const unsigned 
   p.vec_ok = cols % VM_E == 0 && aligned16(out);
   for (int i = 0; i < n_mat; ++i) p.vec_ok = p.vec_ok && aligned16(mat_inputs_host[i]);
   for (int i = 0; i < n_col; ++i) p.vec_ok = p.vec_ok && aligned16(col_inputs_host[i]);
+  // One element a thread where the whole launch then fits the SMs at once and a row is one pass: it is the latency of an
+  // instruction over eight elements that such a launch would wait for.  Also for rows within a warp, which need no more warps
+  // so.  us, layernorm, eight / one: 16 x 33 7.6 / 6.3, 1000 x 128 8.1 / 7.3, 400 x 256 7.0 / 7.0, 1000 x 256 7.2 / 13.4,
+  // 2000 x 33 8.8 / 8.2, 4000 x 33 11.6 / 14.2, 20000 x 8 50 / 32.
   int threads = 32;
-  while (threads < RV_MAX_THREADS && threads * VM_E < cols) threads *= 2;
+  while (threads < RV_MAX_THREADS && threads < cols) threads *= 2;
+  const bool single = cols <= 32 || (cols <= RV_MAX_THREADS && (long)rows * (threads / 32) <= 28L * sm_count());
+  if (!single)
+    for (threads = 32; threads < RV_MAX_THREADS && threads * VM_E < cols;) threads *= 2;
   const int cap = sm_count() * (2048 / threads);
   const size_t smem = (size_t)stack * threads * VM_E * sizeof(float);
   // the limit that needs no opting in, 48 KiB, is on this and the static arrays together
-  if (smem > 46 * 1024) AB200_CUDA(cudaFuncSetAttribute(rowreduce_vm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  rowreduce_vm_kernel<<<rows < cap ? rows : cap, threads, smem, (cudaStream_t)stream>>>(p);
+  auto kern = single ? rowreduce_vm_kernel<1> : rowreduce_vm_kernel<VM_E>;
+  if (smem > 46 * 1024) AB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<rows < cap ? rows : cap, threads, smem, (cudaStream_t)stream>>>(p);
   AB200_CHECK_LAUNCH("rowreduce_vm");
   return AB200_OK;
 }

@@ -130,13 +130,14 @@ inline int vm_translate(const unsigned char *op, const unsigned char *arg, int n
   return e.n;
 }
 
-// VM_E elements of an fp16 / fp32 tensor: element j is i + j * step.  vec: step is 1 and the elements are one
+// E elements (VM_E or 1) of an fp16 / fp32 tensor: element j is i + j * step.  vec: step is 1 and the elements are one
 // aligned chunk; otherwise the first `count` elements exist and the others read as 0.
-__device__ __forceinline__ void vm_load(const void *p, bool f16, size_t i, unsigned step, int count, bool vec, float (&v)[VM_E]) {
-  if (vec) {
+template <int E>
+__device__ __forceinline__ void vm_load(const void *p, bool f16, size_t i, unsigned step, int count, bool vec, float (&v)[E]) {
+  if (E == VM_E && vec) {
     if (f16) {
 #pragma unroll
-      for (int c = 0; c < VM_E / 8; ++c) {
+      for (int c = 0; c < E / 8; ++c) {
         const uint4 h = reinterpret_cast<const uint4 *>(reinterpret_cast<const __half *>(p) + i)[c];
         const uint32_t u[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
@@ -148,36 +149,37 @@ __device__ __forceinline__ void vm_load(const void *p, bool f16, size_t i, unsig
       }
     } else {
 #pragma unroll
-      for (int c = 0; c < VM_E / 4; ++c) {
+      for (int c = 0; c < E / 4; ++c) {
         const float4 a = reinterpret_cast<const float4 *>(reinterpret_cast<const float *>(p) + i)[c];
         v[4 * c] = a.x, v[4 * c + 1] = a.y, v[4 * c + 2] = a.z, v[4 * c + 3] = a.w;
       }
     }
   } else if (f16) {
 #pragma unroll
-    for (int j = 0; j < VM_E; ++j) v[j] = j < count ? __half2float(reinterpret_cast<const __half *>(p)[i + (size_t)j * step]) : 0.f;
+    for (int j = 0; j < E; ++j) v[j] = j < count ? __half2float(reinterpret_cast<const __half *>(p)[i + (size_t)j * step]) : 0.f;
   } else {
 #pragma unroll
-    for (int j = 0; j < VM_E; ++j) v[j] = j < count ? reinterpret_cast<const float *>(p)[i + (size_t)j * step] : 0.f;
+    for (int j = 0; j < E; ++j) v[j] = j < count ? reinterpret_cast<const float *>(p)[i + (size_t)j * step] : 0.f;
   }
 }
-__device__ __forceinline__ void vm_store(void *p, bool f16, size_t i, unsigned step, int count, bool vec, const float (&v)[VM_E]) {
-  if (vec) {
+template <int E>
+__device__ __forceinline__ void vm_store(void *p, bool f16, size_t i, unsigned step, int count, bool vec, const float (&v)[E]) {
+  if (E == VM_E && vec) {
     if (f16) {
       uint4 *o = reinterpret_cast<uint4 *>(reinterpret_cast<__half *>(p) + i);
 #pragma unroll
-      for (int c = 0; c < VM_E / 8; ++c) {
+      for (int c = 0; c < E / 8; ++c) {
         const float *f = v + 8 * c;
         o[c] = make_uint4(h22u(__floats2half2_rn(f[0], f[1])), h22u(__floats2half2_rn(f[2], f[3])), h22u(__floats2half2_rn(f[4], f[5])), h22u(__floats2half2_rn(f[6], f[7])));
       }
     } else {
       float4 *o = reinterpret_cast<float4 *>(reinterpret_cast<float *>(p) + i);
 #pragma unroll
-      for (int c = 0; c < VM_E / 4; ++c) o[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
+      for (int c = 0; c < E / 4; ++c) o[c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < VM_E; ++j)
+    for (int j = 0; j < E; ++j)
       if (j < count) {
         if (f16) reinterpret_cast<__half *>(p)[i + (size_t)j * step] = __float2half_rn(v[j]);
         else reinterpret_cast<float *>(p)[i + (size_t)j * step] = v[j];

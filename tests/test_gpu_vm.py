@@ -39,13 +39,13 @@ def test_elementwise_program_shapes(expr, n):
         assert torch.equal(ops.eltwise_program(prog, consts, [x], out=x), want)  # in place
 
 
-@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 7), (5, 255), (2, 256), (4, 264), (3, 2047), (2, 2048), (3, 2056), (2, 4200), (3000, 33)])
+@pytest.mark.parametrize("rows,cols", [(1, 1), (3, 7), (5, 255), (2, 256), (4, 264), (3, 2047), (2, 2048), (3, 2056), (2, 4200), (3000, 33), (2072, 33), (2073, 33), (4100, 32), (1036, 128), (1037, 127), (518, 256), (519, 256)])
 @pytest.mark.parametrize("dtype", ["float16", "float32"])
 def test_row_programs_at_odd_sizes(rows, cols, dtype):
     text = "m[N] >=! x[N, C]; k[N] <=! x[N, C] * g[C]; s[N] +=! (x[N, C] - m[N]).call(`exp`) * (g[C] + (x[N, C] - k[N]) / (2.0 + g[C])); " \
            "o[N, C] = (x[N, C] - m[N]) / (s[N] + C.val()) + (k[N] - g[C]) * (x[N, C] - w[N, C])"
     dt = getattr(torch, dtype)
-    fn = autort.export(ir=text, inputs=["x=%s[N:4096, C:4200]" % dtype, "w=%s[N:4096, C:4200]" % dtype, "g=%s[C:4200]" % dtype], name="rows_" + dtype)
+    fn = autort.export(ir=text, inputs=["x=%s[N:4200, C:4200]" % dtype, "w=%s[N:4200, C:4200]" % dtype, "g=%s[C:4200]" % dtype], name="rows_" + dtype)
     g = torch.Generator(device="cuda").manual_seed(rows * cols)
     x, w = (torch.randn(rows, cols, generator=g, device="cuda").to(dt) for _ in range(2))
     c = torch.randn(cols, generator=g, device="cuda").abs().to(dt)
